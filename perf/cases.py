@@ -169,3 +169,84 @@ def tolerance(case):
     if case["hidden_bits"] < 32:
         return {"rel": 0.027 if case["kind"] == "dense" else 0.01, "max": 0.2}
     return {"rel": 2e-5, "max": 3e-4} if case["train"] else {"rel": 3e-6, "max": 2e-5}
+
+
+def _fake_quant64(v, scale, top):
+    """Round to the grid and clamp, in 64 bits; the gradient goes straight through inside the range."""
+    q = v / scale
+    code = q.detach().round()
+    inside = (code >= -top) & (code <= top)
+    return (code.clamp(-top, top) + (q - q.detach()) * inside) * scale
+
+
+def _weight64(w, bits):
+    if bits >= 32:
+        return w
+    top = 2 ** (bits - 1) - 1
+    amax = torch.maximum(w.amax(1, keepdim=True).abs(), w.amin(1, keepdim=True).abs())
+    return _fake_quant64(w, amax.clamp(min=1e-8) / top, top)
+
+
+def _hidden64(case, weights):
+    """h [B,H] -> the hidden products [3,B,H] of the gates r, z, n (``weights``: one tensor per gate)."""
+    kind, H = case["kind"], case["H"]
+    if kind == "dense":
+        W = torch.stack([_weight64(w, case["weight_bits"]) for w in weights])
+        return lambda h: torch.matmul(h, W.transpose(1, 2))
+    W = torch.stack(weights)
+    if kind == "diagonal":
+        return lambda h: h * W[:, None, :]
+    if kind == "monarch":
+        def blocks(h):
+            return torch.einsum("bni,gnoi->gbno", h.reshape(h.shape[0], W.shape[1], -1), W).reshape(3, h.shape[0], H)
+        return blocks
+    W = W[:, 0]                                          # [3, factors, log2 n, n/2, 2 (new), 2 (old)]
+    log_n, n = W.shape[2], 2 * W.shape[3]
+
+    def butterfly(h):
+        v = torch.nn.functional.pad(h, (0, n - H)).expand(3, -1, -1)
+        for f in range(W.shape[1]):
+            for s in range(log_n) if f % 2 == 0 else reversed(range(log_n)):
+                stage = s if f % 2 == 0 else log_n - 1 - s
+                tw = W[:, f, stage].reshape(3, 1, n >> (s + 1), 1 << s, 2, 2)
+                old = v.reshape(3, -1, n >> (s + 1), 2, 1 << s)
+                a, b = old[:, :, :, 0], old[:, :, :, 1]
+                v = torch.stack((tw[..., 0, 0] * a + tw[..., 0, 1] * b, tw[..., 1, 0] * a + tw[..., 1, 1] * b), 3)
+                v = v.reshape(3, -1, n)
+        return v[:, :, :H]
+    return butterfly
+
+
+def exact(case, seed):
+    """The same outputs from plain torch operations in 64 bits; none where the states of all steps would not fit."""
+    if case["train"] and case["T"] * case["B"] * case["H"] > 3e8:
+        return None
+    state = prepare(dict(case, graph=False), seed)
+    cell, inputs = state["layer"].cell, [t.double() for t in state["inputs"]]
+    params = [(name, p.detach().double().requires_grad_(case["train"])) for name, p in state["layer"].named_parameters()]
+    by = {name.split(".", 1)[1]: p for name, p in params}
+    scale = {name: float(getattr(cell, name).scale) for name in ("quant_x", "quant_h_in", "quant_h_out")}
+
+    def on_grid(v, name, bits):
+        return v if bits >= 32 else _fake_quant64(v, scale[name], 2 ** (bits - 1) - 1)
+
+    with torch.set_grad_enabled(case["train"]):
+        x = inputs[0].requires_grad_(case["train"] and case["x_grad"])
+        hidden = {"dense": "W_h{}", "diagonal": "struct_Wh_{}.weight", "monarch": "struct_Wh_{}.weight",
+                  "butterfly": "struct_Wh_{}.b.twiddle"}[case["kind"]]
+        product = _hidden64(case, [by[hidden.format(g)] for g in "rzn"])
+        xq = on_grid(x, "quant_x", case["input_bits"])
+        gi = [xq @ _weight64(by[f"W_i{g}"], case["weight_bits"]).t() + by[f"b_i{g}"] for g in "rzn"]
+        h, outs = inputs[1], []
+        for t in range(case["T"]):
+            gh_r, gh_z, gh_n = product(on_grid(h, "quant_h_in", case["hidden_bits"]))
+            r = torch.sigmoid(gi[0][t] + gh_r + by["b_hr"])
+            z = torch.sigmoid(gi[1][t] + gh_z + by["b_hz"])
+            n = torch.tanh(gi[2][t] + r * (gh_n + by["b_hn"]))
+            h = on_grid((1 - z) * n + z * h, "quant_h_out", case["hidden_bits"])
+            outs.append(h)
+        out = torch.stack(outs)
+        if not case["train"]:
+            return out, h
+        wanted = ([x] if case["x_grad"] else []) + [p for _, p in params]
+        return (out.detach(), h.detach(), *torch.autograd.grad(out, wanted, inputs[2]))
