@@ -71,11 +71,55 @@ __global__ void reduce_partials_kernel(const float* __restrict__ src, int nparts
   dst[i] = s;
 }
 
+// Sum of partial vectors, PY partial groups per block: thread (x, y) adds partials y, y + PY, ... of
+// four columns in order and the block adds the PY sums in order, so the result has a fixed order.
+// Memory latency bounds it: the one-thread-per-column loop before kept at most four 4-byte loads in
+// flight (64 partials of 1536 columns: 6 blocks, 18 us); here a column's partials are spread over
+// up to eight threads with up to eight 16-byte loads in flight each.
+template <int PY>
+__global__ void __launch_bounds__(256)
+reduce_partials4_kernel(const float* __restrict__ src, int nparts, size_t row_stride, size_t n, float* __restrict__ dst) {
+  constexpr int PX = 256 / PY;
+  __shared__ float4 part[PY > 1 ? PY : 1][PX];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tx = threadIdx.x % PX, ty = threadIdx.x / PX;
+  const size_t i = ((size_t)blockIdx.x * PX + tx) * 4;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < n) {
+#pragma unroll 8
+    for (int p = ty; p < nparts; p += PY) {
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(src + (size_t)p * row_stride + i));
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+  }
+  if (PY > 1) {
+    part[ty][tx] = s;
+    __syncthreads();
+    if (ty != 0) return;
+#pragma unroll
+    for (int y = 1; y < PY; ++y) {
+      const float4 v = part[y][tx];
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+  }
+  if (i < n) *reinterpret_cast<float4*>(dst + i) = s;
+}
+
 void launch_reduce_partials(const float* src, int nparts, size_t row_stride, size_t n, float* dst,
                             cudaStream_t st) {
-  const unsigned grid = (unsigned)((n + 255) / 256);
-  launch_pdl(reduce_partials_kernel, dim3(grid), dim3(256), 0, st, src, nparts, row_stride, n, dst);
+  const bool vec = n % 4 == 0 && row_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
   note_launch();
+  if (!vec) {
+    launch_pdl(reduce_partials_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
+    return;
+  }
+  // one thread per column group already fills the chip above 2^17 groups; below that the partials are spread
+  const size_t groups = n / 4;
+  if (nparts >= 16 && groups < ((size_t)1 << 14))
+    launch_pdl(reduce_partials4_kernel<8>, dim3((unsigned)((groups + 31) / 32)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
+  else
+    launch_pdl(reduce_partials4_kernel<1>, dim3((unsigned)((groups + 255) / 256)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
 }
 
 // ---------------------------------------------------------------------------
