@@ -155,6 +155,20 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t desc_a, uint64_t 
   }
 }
 
+// One lane of a converged warp.  tcgen05.mma and commit are issued under this predicate and not under
+// `lane == 0`: the compiler then knows that one thread runs the block and keeps the descriptors in
+// uniform registers.  Under a lane test every instruction went through a per-lane broadcast of its
+// operands: 153 cycles per tcgen05.mma at any width, against 128 for the 128x256x16 product itself
+// and 34 for a 64-wide one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
+// Warp index as a value the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // The mbarrier receives one arrival once every tcgen05.mma issued so far by this thread is done.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");

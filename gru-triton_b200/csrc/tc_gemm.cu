@@ -80,7 +80,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __shared__ uint32_t tmem_base_slot;
   __shared__ int dead;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
   const int kb_begin = blockIdx.z * p.kb_per_split;
   const int kb_end = min(p.kb_total, kb_begin + p.kb_per_split);
@@ -121,17 +121,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   GM_MARK(threadIdx.x == 0, 0);      // prologue done
 
   if (warp == 0) {
-    if (lane == 0 && !*deadp) {
-      // ---- loader: one k-block of every plane per stage
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % p.stages, round = i / p.stages;
-        if (round > 0 && !mbar_wait(smem_u32(&bar_empty[s]), (round - 1) & 1, deadp, status)) break;
+    // ---- loader: one k-block of every plane per stage (the whole warp waits, an elected lane issues)
+    bool alive = __all_sync(0xffffffffu, *deadp == 0);
+    int s = 0;
+    uint32_t parity = 1;                                 // the first round finds every stage free
+    for (int i = 0; i < nkb && alive; ++i) {
+      if (i >= p.stages) alive = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_empty[s]), parity, deadp, status));
+      if (!alive) break;
+      if (elect_one()) {
         const uint32_t full = smem_u32(&bar_full[s]);
         mbar_expect_tx(full, (uint32_t)stage_bytes);
-        unsigned char* st = smem + (size_t)s * stage_bytes;
+        const uint32_t st = smem_u32(smem) + (uint32_t)(s * stage_bytes);
         const int kb = kb_begin + i;
         for (int pl = 0; pl < p.a_planes; ++pl) {
-          const uint32_t dst = smem_u32(st + pl * A_PLANE_BYTES);
+          const uint32_t dst = st + (uint32_t)(pl * A_PLANE_BYTES);
           if (A_MN) {
 #pragma unroll
             for (int c = 0; c < BM / 64; ++c)
@@ -140,9 +143,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tma_load_3d(dst, &tmA, kb * KE, m0, pl, full);
           }
         }
-        unsigned char* sb = st + p.a_planes * A_PLANE_BYTES;
+        const uint32_t sb = st + (uint32_t)(p.a_planes * A_PLANE_BYTES);
         for (int pl = 0; pl < p.b_planes; ++pl) {
-          const uint32_t dst = smem_u32(sb + pl * B_PLANE_BYTES);
+          const uint32_t dst = sb + (uint32_t)(pl * B_PLANE_BYTES);
           if (B_MN) {
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
@@ -152,42 +155,52 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
       }
+      __syncwarp();
+      if (++s == p.stages) { s = 0; parity ^= 1u; }
     }
   } else if (warp == 1) {
-    if (lane == 0 && !*deadp) {
-      // ---- issuer.  The fp32 accumulator of the tensor core truncates, so its error grows with
-      // the number of accumulation steps; a chunk of chunk_kb k-blocks is summed in tensor
-      // memory from zero, then handed to the epilogue warps, which keep the running total in
-      // registers with round-to-nearest adds.  Two accumulator buffers alternate.
-      bool alive = true;
-      for (int c = 0; c < nchunks && alive; ++c) {
-        const int buf = c & 1;
-        if (c >= 2 && !mbar_wait(smem_u32(&bar_acc_empty[buf]), ((c >> 1) - 1) & 1, deadp, status)) break;
+    // ---- issuer.  The fp32 accumulator of the tensor core truncates, so its error grows with
+    // the number of accumulation steps; a chunk of chunk_kb k-blocks is summed in tensor
+    // memory from zero, then handed to the epilogue warps, which keep the running total in
+    // registers with round-to-nearest adds.  Two accumulator buffers alternate.
+    // The whole warp walks the ring, one elected lane issues (see elect_one); the descriptors of a
+    // k-block are one base plus constants.
+    constexpr uint64_t A_STEP = (A_MN ? UMMA_K * 128 : 32) >> 4, B_STEP = (B_MN ? UMMA_K * 128 : 32) >> 4;
+    const uint64_t da0 = A_MN ? umma_smem_desc(smem_u32(smem), MN_BK * 128, 1024) : umma_smem_desc(smem_u32(smem), 16, 1024);
+    const uint64_t db0 = B_MN ? umma_smem_desc(smem_u32(smem), MN_BK * 128, 1024) : umma_smem_desc(smem_u32(smem), 16, 1024);
+    const uint32_t b_off = (uint32_t)(p.a_planes * A_PLANE_BYTES) >> 4;
+    bool alive = *deadp == 0;
+    alive = __all_sync(0xffffffffu, alive);
+    int s = 0;
+    uint32_t parity = 0;
+    for (int c = 0; c < nchunks && alive; ++c) {
+      const int buf = c & 1;
+      if (c >= 2) alive = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc_empty[buf]), ((c >> 1) - 1) & 1, deadp, status));
+      if (!alive) break;
+      tc_fence_after();
+      const uint32_t tacc = tmem_acc + (uint32_t)(buf * BN);
+      const int i_begin = c * p.chunk_kb, i_end = min(nkb, (c + 1) * p.chunk_kb);
+      for (int i = i_begin; i < i_end; ++i) {
+        alive = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[s]), parity, deadp, status));
+        if (!alive) break;
         tc_fence_after();
-        const uint32_t tacc = tmem_acc + (uint32_t)(buf * BN);
-        const int i_end = min(nkb, (c + 1) * p.chunk_kb);
-        for (int i = c * p.chunk_kb; i < i_end; ++i) {
-          const int s = i % p.stages, round = i / p.stages;
-          if (!mbar_wait(smem_u32(&bar_full[s]), round & 1, deadp, status)) { alive = false; break; }
-          tc_fence_after();
-          GM_MARK(i == 0, 1);          // first stage landed
-          GM_MARK(i == nkb - 1, 2);    // last stage landed
-          const uint32_t sa = smem_u32(smem + (size_t)s * stage_bytes);
-          const uint32_t sb = sa + p.a_planes * A_PLANE_BYTES;
+        GM_MARK(lane == 0 && i == 0, 1);          // first stage landed
+        GM_MARK(lane == 0 && i == nkb - 1, 2);    // last stage landed
+        if (elect_one()) {
+          const uint32_t st = (uint32_t)(s * stage_bytes) >> 4;
           for (int q = 0; q < p.npairs; ++q) {
-            const uint32_t pa = sa + p.pa[q] * A_PLANE_BYTES, pb = sb + p.pb[q] * B_PLANE_BYTES;
+            const uint64_t da = da0 + st + (uint32_t)(p.pa[q] * (A_PLANE_BYTES >> 4));
+            const uint64_t db = db0 + st + b_off + (uint32_t)(p.pb[q] * (B_PLANE_BYTES >> 4));
+            const uint32_t more = (i > i_begin || q > 0) ? 1u : 0u;
 #pragma unroll
-            for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-              const uint64_t da = A_MN ? umma_smem_desc(pa + kk * UMMA_K * 128, MN_BK * 128, 1024)
-                                       : umma_smem_desc(pa + kk * 32, 16, 1024);
-              const uint64_t db = B_MN ? umma_smem_desc(pb + kk * UMMA_K * 128, MN_BK * 128, 1024)
-                                       : umma_smem_desc(pb + kk * 32, 16, 1024);
-              umma<I8>(tacc, da, db, IDESC, (i > c * p.chunk_kb || q > 0 || kk > 0) ? 1u : 0u);
-            }
+            for (int kk = 0; kk < BK / UMMA_K; ++kk)
+              umma<I8>(tacc, da + kk * A_STEP, db + kk * B_STEP, IDESC, kk > 0 ? 1u : more);
           }
           umma_commit(smem_u32(&bar_empty[s]));          // the stage is free once these MMAs have read it
+          if (i == i_end - 1) umma_commit(smem_u32(&bar_acc_full[buf]));   // this chunk's sum is complete
         }
-        if (alive) umma_commit(smem_u32(&bar_acc_full[buf]));   // this chunk's sum is complete
+        __syncwarp();
+        if (++s == p.stages) { s = 0; parity ^= 1u; }
       }
     }
   } else {

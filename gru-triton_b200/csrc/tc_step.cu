@@ -77,7 +77,7 @@ tc_fwd_step_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __shared__ int dead;
   __shared__ float s_scale[FS_BN], s_bias[FS_BN];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int u0 = blockIdx.x * FS_UNITS, m0 = blockIdx.y * FS_BM;
   const int H = a.H;
   int* status = &g_tc_step_status;
@@ -147,21 +147,24 @@ tc_fwd_step_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
   } else if (warp == 1) {
     pdl_wait();
-    if (lane == 0 && !*deadp) {
-      bool alive = true;
-      for (int i = 0; i < a.nkb && alive; ++i) {
-        const int s = i % FS_STAGES, round = i / FS_STAGES;
-        if (!mbar_wait(smem_u32(&bar_full[s]), round & 1, deadp, status)) { alive = false; break; }
-        tc_fence_after();
-        const uint32_t sa = smem_u32(smem + (size_t)s * FS_STAGE);
-        const uint32_t sb = sa + FS_A_BYTES;
+    // the whole warp walks the ring, one elected lane issues
+    const uint64_t da0 = umma_smem_desc(smem_u32(smem), 16, 1024);
+    const uint64_t db0 = umma_smem_desc(smem_u32(smem) + FS_A_BYTES, 16, 1024);
+    bool alive = __all_sync(0xffffffffu, *deadp == 0);
+    for (int i = 0; i < a.nkb && alive; ++i) {
+      const int s = i % FS_STAGES, round = i / FS_STAGES;
+      alive = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[s]), round & 1, deadp, status));
+      if (!alive) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t st = (uint32_t)(s * FS_STAGE) >> 4;
 #pragma unroll
         for (int kk = 0; kk < FS_KB / 32; ++kk)
-          umma<true>(tmem_acc, umma_smem_desc(sa + kk * 32, 16, 1024), umma_smem_desc(sb + kk * 32, 16, 1024), IDESC,
-                     (i > 0 || kk > 0) ? 1u : 0u);
+          umma<true>(tmem_acc, da0 + st + kk * 2, db0 + st + kk * 2, IDESC, kk > 0 ? 1u : (i > 0 ? 1u : 0u));
         umma_commit(smem_u32(&bar_empty[s]));
+        if (i == a.nkb - 1) umma_commit(smem_u32(&bar_acc));
       }
-      if (alive) umma_commit(smem_u32(&bar_acc));
+      __syncwarp();
     }
   } else {
     pdl_wait();
