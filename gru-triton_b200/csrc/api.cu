@@ -4,12 +4,15 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 
 #include "block_scan.cuh"
 #include "butterfly_scan.cuh"
+#include "tc_cluster.cuh"
 #include "tc_scan.cuh"
 
 namespace b200gru {
@@ -23,9 +26,9 @@ int diag_backward(const float* gi, const float* h0, const float* W, const float*
                   int B, int H, Quant qi, Quant qo, cudaStream_t st);
 
 static std::atomic<unsigned long long> g_launches{0};
-static std::atomic<int> g_test_choice[2] = {{0}, {0}};
+static std::atomic<int> g_test_choice[3] = {{0}, {0}, {0}};
 
-int test_kernel_choice(int slot) { return (slot >= 0 && slot < 2) ? g_test_choice[slot].load(std::memory_order_relaxed) : 0; }
+int test_kernel_choice(int slot) { return (slot >= 0 && slot < 3) ? g_test_choice[slot].load(std::memory_order_relaxed) : 0; }
 static thread_local char g_last_error[256] = {0};
 
 void note_launch(int n) { g_launches.fetch_add((unsigned long long)n, std::memory_order_relaxed); }
@@ -204,6 +207,43 @@ static size_t workspace_bytes(const Dims& d, int backward) {
   return (size_t)-1;
 }
 
+// Kernel of the serial part of a dense / block-diagonal scan: the FP32 cluster kernels or the tensor-core cluster
+// scan, whichever is estimated faster (SM cycles).  Trying every configuration costs tens of microseconds on
+// the host, so the choice is kept per shape (it depends on nothing else); at most 1024 of them.
+struct ScanPlan { bool found, tensor; BlockScanConfig block; tcc::Config tc; };
+
+static ScanPlan plan_scan(const Dims& d, bool fwd, bool w_codes, const Quant& qi) {
+  typedef std::tuple<int, int, int, int, int, int, int> Key;
+  static std::mutex mu;
+  static std::map<Key, ScanPlan> cache;
+  const int forced = test_kernel_choice(2);
+  const int h_codes = qi.enabled && qi.qmin >= -128.f && qi.qmax <= 127.f;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const Key key(dev, d.T, d.B, d.Hb, d.nb, (fwd ? 1 : 0) | (w_codes ? 2 : 0) | (h_codes ? 4 : 0), forced);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) return it->second;
+  }
+  ScanPlan p;
+  memset(&p, 0, sizeof(p));
+  double block_cycles = 0.0, tc_cycles = 0.0;
+  const bool block = choose_block_config(fwd, d.T, d.B, d.Hb, d.nb, &p.block, &block_cycles);
+  const bool tensor = forced != 1 && tcc::choose(fwd, d.T, d.B, d.Hb, d.nb, w_codes, qi, &p.tc, &tc_cycles);
+  p.found = block || tensor;
+  p.tensor = tensor && (forced == 2 || !block || tc_cycles < block_cycles);
+  static const bool debug = getenv("B200GRU_DEBUG") != nullptr;
+  if (debug)
+    fprintf(stderr, "[b200gru] %s T=%d B=%d H=%d nb=%d: tensor-core cluster scan C=%d N=%d rows=%d active=%d %.0f cycles, "
+            "FP32 clusters %.0f\n", fwd ? "forward" : "backward", d.T, d.B, d.H, d.nb, p.tc.C, p.tc.N, p.tc.rows, p.tc.active,
+            tc_cycles, block_cycles);
+  std::lock_guard<std::mutex> lk(mu);
+  if (cache.size() >= 1024) cache.clear();
+  cache[key] = p;
+  return p;
+}
+
 static int fill_bfly(const Dims& d, BflyArgs* a) {
   memset(a, 0, sizeof(*a));
   a->T = d.T; a->B = d.B; a->H = d.H; a->Hpad = d.Hpad; a->logn = d.logn; a->nstages = d.nstages;
@@ -256,8 +296,17 @@ static int scan_forward_impl(const b200gru_shape* shape, const float* gi, const 
         const tc::TcWeights w = {W, codes, scales};
         return tc::launch_tc_dense_forward(gi, h0, w, bh, out, save, workspace, d.T, d.B, d.H, qi, qo, st);
       }
-      BlockScanConfig cfg;
-      if (!choose_block_config(true, d.B, d.Hb, d.nb, &cfg)) return B200GRU_UNSUPPORTED;
+      const ScanPlan plan = plan_scan(d, true, codes != nullptr && scales != nullptr, qi);
+      if (!plan.found) return B200GRU_UNSUPPORTED;
+      if (plan.tensor) {
+        tcc::Args t;
+        memset(&t, 0, sizeof(t));
+        t.gi = gi; t.h0 = h0; t.W = W; t.codes = codes; t.scales = scales; t.bh = bh; t.out = out; t.save = save;
+        t.T = d.T; t.B = d.B; t.H = d.H; t.nb = d.nb; t.Hb = d.Hb;
+        t.w_gate_stride = d.gate_stride; t.w_block_stride = d.block_stride; t.qin = qi; t.qout = qo;
+        return tcc::launch(true, plan.tc, t, st);
+      }
+      const BlockScanConfig& cfg = plan.block;
       BlockScanArgs a;
       memset(&a, 0, sizeof(a));
       a.gi = gi; a.h0 = h0; a.W = W; a.bh = bh; a.out = out; a.save = save;
@@ -340,16 +389,27 @@ static int scan_backward_impl(const b200gru_shape* shape, const float* gi, const
         return tc::launch_tc_dense_backward(h0, w, out, S, dout, dgi, dh0, dW, dbh, ws + s_off, d.T, d.B, d.H, qi, qo,
                                             st);
       }
-      BlockScanConfig cfg;
-      if (!choose_block_config(false, d.B, d.Hb, d.nb, &cfg)) return B200GRU_UNSUPPORTED;
-      BlockScanArgs a;
-      memset(&a, 0, sizeof(a));
-      a.gi = gi; a.h0 = h0; a.W = W; a.bh = bh; a.out = const_cast<float*>(out); a.S = S; a.dout = dout;
-      a.dgi = dgi; a.dh0 = dh0;
-      a.T = d.T; a.B = d.B; a.H = d.H; a.nb = d.nb; a.Hb = d.Hb;
-      a.w_gate_stride = d.gate_stride; a.w_block_stride = d.block_stride;
-      a.qin = qi; a.qout = qo;
-      int rc = launch_block_scan(false, cfg, a, d.nb, st);
+      const ScanPlan plan = plan_scan(d, false, codes != nullptr && scales != nullptr, qi);
+      if (!plan.found) return B200GRU_UNSUPPORTED;
+      int rc;
+      if (plan.tensor) {
+        tcc::Args t;
+        memset(&t, 0, sizeof(t));
+        t.h0 = h0; t.W = W; t.codes = codes; t.scales = scales; t.out = const_cast<float*>(out); t.S = S; t.dout = dout;
+        t.dgi = dgi; t.dh0 = dh0;
+        t.T = d.T; t.B = d.B; t.H = d.H; t.nb = d.nb; t.Hb = d.Hb;
+        t.w_gate_stride = d.gate_stride; t.w_block_stride = d.block_stride; t.qin = qi; t.qout = qo;
+        rc = tcc::launch(false, plan.tc, t, st);
+      } else {
+        BlockScanArgs a;
+        memset(&a, 0, sizeof(a));
+        a.gi = gi; a.h0 = h0; a.W = W; a.bh = bh; a.out = const_cast<float*>(out); a.S = S; a.dout = dout;
+        a.dgi = dgi; a.dh0 = dh0;
+        a.T = d.T; a.B = d.B; a.H = d.H; a.nb = d.nb; a.Hb = d.Hb;
+        a.w_gate_stride = d.gate_stride; a.w_block_stride = d.block_stride;
+        a.qin = qi; a.qout = qo;
+        rc = launch_block_scan(false, plan.block, a, d.nb, st);
+      }
       if (rc) return rc;
       if (tc_wgrad_path(d)) {
         // off-chain products on the tensor cores: bias sums first (their scratch leads), then dW
@@ -523,6 +583,8 @@ int b200gru_dense_q8_backward(const float* gi, const float* h0, const float* Wq,
   return scan_backward_impl(&s, gi, h0, Wq, codes, scales, bh_cat, out, dout, save, q_in, q_out, dgi, dh0, dWq, dbh,
                             workspace, workspace_bytes_, stream);
 }
+
+void b200gru_test_select_dense_scan(int which) { g_test_choice[2].store(which, std::memory_order_relaxed); }
 
 void b200gru_test_select_kernels(int butterfly_register_kernels, int diagonal_register_ring) {
   g_test_choice[0].store(butterfly_register_kernels, std::memory_order_relaxed);

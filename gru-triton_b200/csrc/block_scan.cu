@@ -41,6 +41,7 @@
 #include <tuple>
 
 #include "block_scan.cuh"
+#include "tc_cluster.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -935,8 +936,8 @@ static int* scan_status_address() {
 }
 
 // Pick the cluster size, batch tile and weight placement that minimise a simple cost model:
-//   step = max(FMA issue, shared-memory streaming) + barrier;  total = waves * step.
-bool choose_block_config(bool fwd, int B, int Hb, int nb, BlockScanConfig* out) {
+//   step = contraction (FMA issue, shared-memory streaming) + latency + exchange;  total = waves * steps.
+bool choose_block_config(bool fwd, int T, int B, int Hb, int nb, BlockScanConfig* out, double* cycles) {
   const DeviceInfo di = device_info();
   if (!di.ok) return false;
   double best = 1e300;
@@ -990,15 +991,26 @@ bool choose_block_config(bool fwd, int B, int Hb, int nb, BlockScanConfig* out) 
         if (active <= 0) continue;
         const long long nclusters = (long long)nb * cdiv(B, BT);
         const double waves = (double)((nclusters + active - 1) / active);
+        // Cycles of a step, fitted to measurements at Hb = 64 .. 512 and BT = 1 .. 5 (Hb = 512, C = 16: forward 3040 at
+        // BT = 1, 6360 at 5; backward 3800 and 6760).  The forward adds a latency per item (four units of a warp): a CTA
+        // that owns 128 units of Hb = 128 by itself took 7700 cycles where four CTAs of 32 units take 1570.
         const double fma = 3.0 * Hc4 * Hb * BT / 128.0;
-        const double stream = 3.0 * Hc4 * Hb * 4.0 / (ws ? 128.0 : 24.0) + (double)Hb * BT * 4.0 * NW / 128.0;
-        const double barrier = C > 1 ? 1200.0 + 40.0 * C : 200.0;
-        const double cost = waves * ((fma > stream ? fma : stream) + barrier + 400.0);
+        const double wstream = 3.0 * Hc4 * Hb * 4.0 / (ws ? 128.0 : 24.0), hstream = (double)Hb * BT * 4.0 * NW / 128.0;
+        double step;
+        if (fwd) {
+          step = 0.6 * wstream + fma + hstream + (200.0 + 290.0 * BT) * ipw + (C > 1 ? 700.0 + 40.0 * C : 1000.0);
+        } else {
+          const double barrier = C > 1 ? 1200.0 + 40.0 * C : 1400.0;
+          step = (fma > wstream + hstream ? fma : wstream + hstream) + barrier + 400.0;
+          step += c.TW == 1 ? 45.0 * Hc4 * (BT - 1) / c.NH : 0.11 * (BT - 1) * step;
+        }
+        const double cost = waves * (step + 25000.0 / T);
         if (cost < best) { best = cost; found = true; *out = c; }
         break;                                          // weights in smem fit: do not also try global
       }
     }
   }
+  *cycles = best * T;
   return found;
 }
 
@@ -1041,8 +1053,9 @@ extern "C" int b200gru_device_status(int reset) {
   const int f = bfly_read_status(reset);
   const int g = tc::tc_read_status(reset);
   const int s = tc::tc_step_read_status(reset);
-  if (d < 0 || f < 0 || g < 0 || s < 0) return -1;
-  return (v != 0 || d != 0 || f != 0 || g != 0 || s != 0) ? 1 : 0;
+  const int c = tcc::read_status(reset);
+  if (d < 0 || f < 0 || g < 0 || s < 0 || c < 0) return -1;
+  return (v != 0 || d != 0 || f != 0 || g != 0 || s != 0 || c != 0) ? 1 : 0;
 }
 
 }  // namespace b200gru

@@ -44,7 +44,8 @@ struct BlockScanConfig {
 // cluster sizes; the forward reads 4 units at a time and may run past the last owned unit).
 inline int transposed_row_bound(int Hb) { return Hb + 72; }     // C * round_up(ceil(Hb / C), 4) + 4 + 4, C <= 16
 
-bool choose_block_config(bool fwd, int B, int Hb, int nb, BlockScanConfig* out);
+// *cycles: estimated SM cycles of the scan with the configuration chosen.
+bool choose_block_config(bool fwd, int T, int B, int Hb, int nb, BlockScanConfig* out, double* cycles);
 int launch_block_scan(bool fwd, const BlockScanConfig& c, BlockScanArgs args, int nb, cudaStream_t st);
 
 // block_gemm.cu -- the parallel (off-chain) parts of the dense / block-diagonal backward.

@@ -170,7 +170,8 @@ int tc_step_read_status(int reset);  // fused tensor-core step (tc_step.cu)
 
 // Test hook (b200gru_test_select_kernels): slot 0 != 0 -> butterfly launches use the register /
 // global-twiddle kernels on every shape; slot 1 != 0 -> the diagonal forward uses the register-ring
-// kernel on every shape.  Defaults 0: the dispatch is by shape only.
+// kernel on every shape.  Slot 2 (b200gru_test_select_dense_scan): 1 -> FP32 cluster kernels, 2 -> tensor-core
+// cluster scan wherever it applies.  Defaults 0: the dispatch is by shape only.
 int test_kernel_choice(int slot);
 
 // Launch bookkeeping shared by all translation units (defined in api.cu).

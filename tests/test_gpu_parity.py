@@ -117,6 +117,53 @@ def test_scan_parity(kind, T, B, H, quant):
 
 
 @pytest.mark.parametrize("quant", [None, Q8], ids=["fp32", "q8"])
+@pytest.mark.parametrize("T,B,H,nb", [(1, 1, 32, 1), (3, 5, 96, 1), (5, 3, 33, 1), (4, 17, 129, 1), (3, 48, 256, 1),
+                                      (2, 49, 257, 1), (9, 33, 512, 1), (3, 300, 512, 1), (4, 20, 192, 4), (3, 9, 66, 2)])
+def test_tensor_core_cluster_scan(T, B, H, nb, quant):
+    """The tensor-core cluster scan at the edges of its tiles: one CTA to sixteen, 32-unit slabs that are full or
+    hold one unit, row tiles of 16 / 32 / 48 that are full, short or many; held to the same bars as the FP32
+    kernels (its operands carry 22 significant bits, 2^-23 of a term, below the 1e-5 / 1e-4 of the parity tests)."""
+    from gru_triton_b200 import _lib
+    kind = "dense" if nb == 1 else "monarch"
+    fwd, bwd, _ = _mods()[kind]
+    gi, h0, W, bh, dout = orc.make_problem(kind, T, B, H, seed=11 + T + B + H, **({} if nb == 1 else {"nblocks": nb}))
+    if quant is None and B == 5:
+        # A state outside the unit range takes a scale of its own.  |h0| <= 4: a pre-activation is off by at most
+        # 2^-23 * sum |w||h| = 2^-23 * 96 * 0.05 * 4 = 2.3e-6 and moves h by |h0| / 4 of that, inside the 1e-5 bar; at
+        # |h0| = 1000 the blend itself amplifies the rounding of any fp32 sum beyond it.
+        h0 = h0 * (4.0 / float(h0.abs().max()))
+    kw = dict(h_in_quant=quant[0], h_out_quant=quant[1]) if quant else {}
+    d = _cuda(gi, h0, W, bh, dout)
+    _lib.load().b200gru_test_select_dense_scan(2)
+    try:
+        out = fwd(*d[:4], **kw)
+        grads = bwd(*d[:4], out, d[4], **kw)
+        torch.cuda.synchronize()
+    finally:
+        _lib.load().b200gru_test_select_dense_scan(0)
+    check_forward(kind, out, gi, h0, W, bh, quant)
+    check_backward(kind, grads, gi, h0, W, bh, out, dout, quant)
+
+
+@pytest.mark.parametrize("T,B,H", [(3, 5, 96), (4, 40, 512)])
+def test_tensor_core_cluster_scan_weight_codes(T, B, H):
+    """The same with int8 weight codes and an int8 state: products of integer codes, exact in the accumulator."""
+    from gru_triton_b200 import _lib
+    gi, h0, W, bh, dout = orc.make_problem("dense", T, B, H, seed=5 + H)
+    d = _cuda(gi, h0, W, bh, dout)
+    codes, scales, Wq = _lib.quantize_rows(d[2], 8)
+    _lib.load().b200gru_test_select_dense_scan(2)
+    try:
+        out, save = _lib.scan_forward("dense", d[0], d[1], Wq, d[3], *Q8, want_save=True, codes=codes, scales=scales)
+        grads = _lib.scan_backward("dense", d[0], d[1], Wq, d[3], out, d[4], save, *Q8, codes=codes, scales=scales)
+        torch.cuda.synchronize()
+    finally:
+        _lib.load().b200gru_test_select_dense_scan(0)
+    check_forward("dense", out, gi, h0, Wq.cpu(), bh, Q8)
+    check_backward("dense", grads, gi, h0, Wq.cpu(), bh, out, dout, Q8)
+
+
+@pytest.mark.parametrize("quant", [None, Q8], ids=["fp32", "q8"])
 @pytest.mark.parametrize("T,B,H,extra", [(8, 4, 32, {}), (16, 32, 512, {}), (5, 3, 48, {"butterfly_nblocks": 2}),
                                          (3, 2, 1024, {})])
 def test_butterfly_alternate_kernels(T, B, H, extra, quant):
