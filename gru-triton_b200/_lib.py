@@ -80,6 +80,9 @@ SIGNATURES = {
     "b200gru_calibration_workspace_bytes": (_Z, [_SP]),
     "b200gru_calibration_scan": (_I, [_SP, _P, _P, _P, _P, _I, ctypes.c_double, _P, _P, _I, _P, _P, _I, _P, _P, _Z, _P]),
     "b200gru_device_status": (_I, [_I]),
+    "b200gru_layer_sizes": (_I, [_P, _P]),
+    "b200gru_layer_forward": (_I, [_P, _P, _P, _P]),
+    "b200gru_layer_backward": (_I, [_P, _P, _P, _P]),
     "b200gru_test_select_kernels": (None, [_I, _I]),
     "b200gru_test_select_dense_scan": (None, [_I]),
     "b200gru_test_wait_timeout": (_I, [_P]),

@@ -121,6 +121,15 @@ __device__ __forceinline__ float ste_mask(float x, const Quant& q) {
   return (c >= q.qmin && c <= q.qmax) ? 1.0f : 0.0f;
 }
 
+// Power of two s with mx * s in [2^14, 2^15) and its inverse, both normal numbers; 1 for zero, infinities and NaN.
+__device__ __forceinline__ void pow2_row_scale(float mx, float* s, float* inv) {
+  int e = (int)((__float_as_uint(mx) >> 23) & 0xffu) - 127;       // floor(log2 mx)
+  if (!(mx > 0.f) || e > 127) { *s = 1.f; *inv = 1.f; return; }
+  e = 14 - max(-100, e);
+  *s = __uint_as_float((uint32_t)(127 + e) << 23);
+  *inv = __uint_as_float((uint32_t)(127 - e) << 23);
+}
+
 struct GateOut {
   float r, z, n, h_raw;
 };

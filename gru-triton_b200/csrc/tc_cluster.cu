@@ -133,14 +133,6 @@ __device__ __forceinline__ void wait_cluster(uint32_t bar, uint32_t parity, vola
 __device__ __forceinline__ void bar_compute() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); }
 __device__ __forceinline__ void bar_all() { asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory"); }
 
-// Power of two s with mx * s in [2^14, 2^15), and its inverse; 1 for zero, infinities and NaN.
-__device__ __forceinline__ void pow2_scale(float mx, float* s, float* inv) {
-  int e = (int)((__float_as_uint(mx) >> 23) & 0xffu) - 127;       // floor(log2 mx)
-  if (!(mx > 0.f) || e > 127) { *s = 1.f; *inv = 1.f; return; }
-  e = 14 - max(-100, e);
-  *s = __uint_as_float((uint32_t)(127 + e) << 23);
-  *inv = __uint_as_float((uint32_t)(127 - e) << 23);
-}
 __device__ __forceinline__ float warp_max(float v) {              // v >= 0 (or NaN, which counts as largest)
   return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
 }
@@ -290,7 +282,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
         for (int q = 0; q < 4; ++q)
 #pragma unroll
           for (int e = 0; e < 4; ++e) mx = fmaxf(mx, fabsf(v[q][e]));
-        pow2_scale(warp_max(mx), &s, &inv);
+        pow2_row_scale(warp_max(mx), &s, &inv);
       } else {
         inv = own ? a.scales[g * H + u0 + j] : 0.f;
       }
@@ -349,7 +341,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
         mx = fmaxf(1.f, warp_max(mx));
         if (a.qin.enabled) mx += a.qin.scale;
         if (a.qout.enabled) mx += a.qout.scale;
-        pow2_scale(mx, &s, &inv);
+        pow2_row_scale(mx, &s, &inv);
         if (lane == 0) { s_h[b] = s; s_inv_h[b] = inv; }
       }
       for (int slot = 0; slot < CS; ++slot) {
@@ -602,7 +594,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
           const float* src = a.W + (size_t)g * a.w_gate_stride + (size_t)n * a.w_block_stride + (size_t)(u0 + j) * Hb;
           for (int k = lane; k < Hb; k += 32) mx = fmaxf(mx, fabsf(__ldg(src + k)));
         }
-        pow2_scale(warp_max(mx), &s, &inv);
+        pow2_row_scale(warp_max(mx), &s, &inv);
       } else {
         inv = own ? a.scales[g * H + u0 + j] : 0.f;
       }
@@ -770,7 +762,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
         // operand planes, scaled by a power of two of this row's largest entry
         const float vr = gr[i] * fr, vz = gz[i] * fz, vn = gg.dghn * fn;
         float s, inv;
-        pow2_scale(warp_max(fmaxf(fabsf(vr), fmaxf(fabsf(vz), fabsf(vn)))), &s, &inv);
+        pow2_row_scale(warp_max(fmaxf(fabsf(vr), fmaxf(fabsf(vz), fabsf(vn)))), &s, &inv);
         const int b = warp + NW * i;
         if (lane == 0) s_inv[it & 1][b] = inv;
         unsigned char* dst = bop + sw64((uint32_t)b, lane * 2);

@@ -375,15 +375,14 @@ split_planes_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ d
   }
 }
 
-// Two fp16 planes of every row of src[rows][cols], scaled by a power of two of the row's own:
-// s_r = 2^(15 - e) with max|row| = m * 2^e, m in [0.5, 1), so the largest scaled element lies in
-// [2^14, 2^15).  hi = RN16(x * s), lo = RN16(x * s - hi) (the difference is exact in fp32), and
-// inv_scale[r] = 1 / s_r exactly.  hi + lo carries 22 significant bits of every element that is
-// not below 2^-17 of its row's largest; smaller ones keep an absolute error of 2^-40 of it.
-// One warp per row; the second read of the row hits L1.
+// Two fp16 planes of every row of src[rows][cols] (times col_scale[cols] when given), scaled by a power of
+// two of the row's own so that its largest element lies in [2^14, 2^15).  hi = RN16(x * s), lo = RN16(x * s - hi)
+// (the difference is exact in fp32), and inv_scale[r] = 1 / s_r exactly.  hi + lo carries 22 significant
+// bits of every element that is not below 2^-17 of its row's largest; smaller ones keep an absolute
+// error of 2^-40 of it.  One warp per row; the second read of the row hits L1.
 __global__ void __launch_bounds__(256)
 split_rows_f16_kernel(const float* __restrict__ src, __half* __restrict__ dst, int rows, int cols, size_t plane_stride,
-                      float* __restrict__ inv_scale) {
+                      float* __restrict__ inv_scale, const float* __restrict__ col_scale) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -391,25 +390,29 @@ split_rows_f16_kernel(const float* __restrict__ src, __half* __restrict__ dst, i
   if (row >= rows) return;
   const float4* s4 = reinterpret_cast<const float4*>(src + (size_t)row * cols);
   const int c4 = cols >> 2;
+  auto load = [&](int i) {
+    float4 v = s4[i];
+    if (col_scale != nullptr) {
+      const float4 c = __ldg(reinterpret_cast<const float4*>(col_scale) + i);
+      v.x *= c.x; v.y *= c.y; v.z *= c.z; v.w *= c.w;
+    }
+    return v;
+  };
   float mx = 0.f;
+#pragma unroll 4
   for (int i = lane; i < c4; i += 32) {
-    const float4 v = s4[i];
+    const float4 v = load(i);
     mx = fmaxf(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))), mx);
   }
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  int e = 0;
-  float s = 1.0f, inv = 1.0f;
-  if (mx > 0.f && mx < 3.0e38f) {
-    frexpf(mx, &e);
-    e = max(-110, min(110, e));               // both 2^(15-e) and 2^(e-15) stay normal
-    s = ldexpf(1.0f, 15 - e);
-    inv = ldexpf(1.0f, e - 15);
-  }
+  float s, inv;
+  pow2_row_scale(mx, &s, &inv);
   if (lane == 0) inv_scale[row] = inv;
   __half* d = dst + (size_t)row * cols;
+#pragma unroll 4
   for (int i = lane; i < c4; i += 32) {
-    const float4 v = s4[i];
+    const float4 v = load(i);
     const float x[4] = {v.x * s, v.y * s, v.z * s, v.w * s};
     __half hi[4], lo[4];
 #pragma unroll
@@ -646,17 +649,22 @@ int launch_split_planes(const float* src, void* dst, size_t n, size_t plane_stri
   return check_launch("split_planes_kernel");
 }
 
-int launch_split_rows_f16(const float* src, void* dst, int rows, int cols, size_t plane_stride, float* inv_scale,
-                          cudaStream_t st) {
+int launch_split_rows_f16_scaled(const float* src, void* dst, int rows, int cols, size_t plane_stride, float* inv_scale,
+                                 const float* col_scale, cudaStream_t st) {
   if (src == nullptr || dst == nullptr || inv_scale == nullptr || rows < 0 || cols <= 0 || (cols & 3) ||
       (plane_stride & 3))
     return B200GRU_INVALID_ARGUMENT;
-  if (!aligned16(src) || (reinterpret_cast<uintptr_t>(dst) & 7u)) return B200GRU_INVALID_ARGUMENT;
+  if (!aligned16(src) || (reinterpret_cast<uintptr_t>(dst) & 7u) || !aligned16(col_scale)) return B200GRU_INVALID_ARGUMENT;
   if (rows == 0) return B200GRU_OK;
   launch_pdl(split_rows_f16_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st, src, static_cast<__half*>(dst),
-             rows, cols, plane_stride, inv_scale);
+             rows, cols, plane_stride, inv_scale, col_scale);
   note_launch();
   return check_launch("split_rows_f16_kernel");
+}
+
+int launch_split_rows_f16(const float* src, void* dst, int rows, int cols, size_t plane_stride, float* inv_scale,
+                          cudaStream_t st) {
+  return launch_split_rows_f16_scaled(src, dst, rows, cols, plane_stride, inv_scale, nullptr, st);
 }
 
 }  // namespace tc

@@ -61,5 +61,9 @@ int launch_split_planes(const float* src, void* dst, size_t n, size_t plane_stri
 int launch_split_rows_f16(const float* src, void* dst, int rows, int cols, size_t plane_stride, float* inv_scale,
                           cudaStream_t st);
 
+// The same of src * col_scale[cols] (16-byte aligned).
+int launch_split_rows_f16_scaled(const float* src, void* dst, int rows, int cols, size_t plane_stride, float* inv_scale,
+                                 const float* col_scale, cudaStream_t st);
+
 }  // namespace tc
 }  // namespace b200gru

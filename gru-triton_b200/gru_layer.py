@@ -35,6 +35,8 @@ def _extract_h_quant_params(quantizer: FakeQuantize):
     replaced or written, so a frozen layer's forward neither synchronises nor breaks a CUDA-graph
     capture."""
     cfg = quantizer.config
+    if type(quantizer) is Identity:
+        return None
     if cfg.mode != "frozen" or not isinstance(quantizer, FakeQuantizePerTensor) or not cfg.symmetric:
         return None
     scale = quantizer.scale
@@ -202,8 +204,12 @@ class GRULayer(nn.Module):
 
     def _forward_fast_dispatch(self, x, h0):
         """Input projection hoisted to one GEMM, then the persistent CUDA scan
-        (gru_layer.py:234-302)."""
+        (gru_layer.py:234-302); one library call where the layer has the common form."""
         cell = self.cell
+        from . import layer_native
+        out = layer_native.forward(self, x, h0)
+        if out is not None:
+            return (out.transpose(0, 1) if self.batch_first else out), out[-1]
         if cell._input_dense:
             gi = self._input_projection_fast(x)
         else:

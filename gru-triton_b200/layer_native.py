@@ -1,0 +1,230 @@
+"""Layer calls through one library entry per direction (``b200gru_layer_forward`` / ``_backward``).
+
+``forward(layer, x, h0)`` runs the input projection and the scan of a dispatchable ``GRULayer`` with
+a dense input side and returns ``out``, or ``None`` where the call has a form this path does not take
+(other dtypes or devices, widths that are no multiple of 8, quantizers other than the kinds the
+kernels implement, tracing and function transforms): the caller then goes through the composed path
+of ``tc.linear`` and the scan functions, which also words the errors.
+
+One step of one sequence (T = B = 1, 256 x 256) spent 190 us in the composed path's Python: four
+concatenations, two autograd functions and a dozen library calls around 23 us of kernels.
+"""
+
+from __future__ import annotations
+
+import ctypes
+from functools import lru_cache
+
+import torch
+
+from . import _lib
+from .quantizers import FakeQuantizePerChannel, Identity
+
+_TRAIN, _DX, _DWI, _DBI = 1, 2, 4, 8
+_INTS = ctypes.c_int * 10
+_FLOATS = ctypes.c_float * 12
+_FWD_PTRS = ctypes.c_void_p * 18
+_BWD_PTRS = ctypes.c_void_p * 13
+_SIZES = ctypes.c_size_t * 3
+_GATES = "rzn"
+
+
+@lru_cache(maxsize=512)
+def _plan(kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h, flags):
+    """``(dims, kept bytes, forward scratch, backward scratch)`` of a shape, or None if it has none."""
+    dims = _INTS(_lib.KIND[kind], T, B, I, H, nblocks, log2_hpad, bits_i, bits_h, flags)
+    sizes = _SIZES()
+    if _lib.load().b200gru_layer_sizes(dims, sizes):
+        return None
+    return (dims, *sizes)
+
+
+@lru_cache(maxsize=512)
+def _quants(qx, qi, qo):
+    vals = []
+    for q in (qx, qi, qo):
+        vals += [1.0, 0.0, 0.0, 0.0] if q is None else [q[0], q[1], q[2], 1.0]
+    return _FLOATS(*vals)
+
+
+def _weight_bits(quantizers):
+    """Bit width the weight-preparation kernel implements for these three quantizers (32: identities), else None."""
+    a, b, c = quantizers
+    if type(a) is Identity and type(b) is Identity and type(c) is Identity:
+        return 32
+    bits = a.config.bits
+    for q in quantizers:
+        cfg = q.config
+        if (not isinstance(q, FakeQuantizePerChannel) or cfg.axis != 0 or not cfg.symmetric or cfg.mode != "dynamic" or
+                cfg.bits != bits or bits > 8):
+            return None
+    return int(bits)
+
+
+def _plain(t, shape, device):
+    return ((type(t) is torch.nn.Parameter or type(t) is torch.Tensor) and t.dtype is torch.float32 and
+            t.device == device and t.shape == shape and t.is_contiguous())
+
+
+def _transformed() -> bool:
+    """Function transforms, forward-mode AD and tracing look at every operation: not for one opaque call."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or
+            torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing() or torch.compiler.is_compiling())
+
+
+def _parameters(cell, kind, device, I, H):
+    """``(params, nblocks, log2_hpad)``: input weights, hidden weights, input biases, hidden biases per gate."""
+    own, mods = cell._parameters, cell._modules
+    wi = [own.get("W_i" + g) for g in _GATES]
+    nblocks, log2_hpad = 1, 0
+    if kind == "dense":
+        wh, shape = [own.get("W_h" + g) for g in _GATES], (H, H)
+    else:
+        structs = [mods["struct_Wh_" + g] for g in _GATES]
+        if kind == "butterfly":
+            wh = [s.b.twiddle for s in structs]
+            shape = wh[0].shape
+            if len(shape) != 6 or shape[0] != 1 or 2 * shape[3] != 1 << shape[2] or 2 * shape[3] < H or tuple(shape[4:]) != (2, 2):
+                return None
+            nblocks, log2_hpad = shape[1], shape[2]
+        else:
+            wh = [s.weight for s in structs]
+            if kind == "diagonal":
+                shape = (H,)
+            else:
+                nblocks = wh[0].shape[0]
+                if nblocks == 0 or H % nblocks:
+                    return None
+                shape = (nblocks, H // nblocks, H // nblocks)
+    biases = [own.get("b_" + s + g) for s in "ih" for g in _GATES]
+    if any(b is None for b in biases):
+        if any(b is not None for b in biases) or any(getattr(cell, "b_" + s + g, None) is not None for s in "ih" for g in _GATES):
+            return None
+        biases = None
+    elif not all(_plain(b, (H,), device) for b in biases):
+        return None
+    if not (all(_plain(w, (H, I), device) for w in wi) and all(_plain(w, shape, device) for w in wh)):
+        return None
+    return wi + wh + (biases or []), nblocks, log2_hpad
+
+
+def _addresses(params):
+    ptrs = [p.data_ptr() for p in params]
+    return ptrs if len(ptrs) == 12 else ptrs + [None] * 6
+
+
+def _run(x, h0, key, quants, params, train):
+    plan = _plan(*key)
+    dims, kept_bytes, scratch_bytes, _ = plan
+    kind, T, B, I, H = key[:5]
+    device = x.device
+    out = torch.empty((T, B, H), device=device, dtype=torch.float32)
+    save = None
+    if train:
+        save = torch.empty((T, B, 3 * H) if kind == "diagonal" else (4, T, B, H), device=device, dtype=torch.float32)
+    kept = torch.empty(kept_bytes, device=device, dtype=torch.uint8)
+    scratch = torch.empty(scratch_bytes, device=device, dtype=torch.uint8)
+    ptrs = _FWD_PTRS(x.data_ptr(), h0.data_ptr(), *_addresses(params), out.data_ptr(), None if save is None else save.data_ptr(),
+                     kept.data_ptr(), scratch.data_ptr())
+    rc = _call(_lib.load().b200gru_layer_forward, dims, quants, ptrs, device)
+    if rc:
+        _lib._raise(rc, f"{kind} layer forward")
+    _lib._after_call()
+    return out, save, kept
+
+
+def _call(fn, dims, quants, ptrs, device):
+    index = device.index
+    if torch._C._cuda_getDevice() == index:
+        return fn(dims, quants, ptrs, torch._C._cuda_getCurrentRawStream(index))
+    with torch.cuda.device(index):
+        return fn(dims, quants, ptrs, torch._C._cuda_getCurrentRawStream(index))
+
+
+class LayerFunction(torch.autograd.Function):
+    """``out[T,B,H]`` of a layer call; ``params`` as :func:`_parameters` lists them."""
+
+    @staticmethod
+    def forward(ctx, x, h0, key, quants, *params):
+        train = any(ctx.needs_input_grad)
+        out, save, kept = _run(x, h0, key[:9] + (_TRAIN if train else 0,), quants, params, train)
+        ctx.key, ctx.quants, ctx.nparams = key, quants, len(params)
+        if train:
+            ctx.save_for_backward(x, h0, out, save, kept)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        x, h0, out, save, kept = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        kind, T, B, I, H, nblocks, log2_hpad = ctx.key[:7]
+        has_bias = ctx.nparams == 12
+        want_dx, want_wi, want_bi = need[0], any(need[4:7]), has_bias and any(need[10:13])
+        dims, _, _, scratch_bytes = _plan(*ctx.key[:9], _TRAIN)
+        device = x.device
+        dout = dout.contiguous()
+        dx = torch.empty_like(x) if want_dx else None
+        dh0 = torch.empty_like(h0)
+        dwi = torch.empty((3, H, I), device=device, dtype=torch.float32) if want_wi else None
+        shape = {"dense": (H, H), "diagonal": (H,), "monarch": (nblocks, H // nblocks, H // nblocks),
+                 "butterfly": (1, nblocks, log2_hpad, (1 << log2_hpad) // 2, 2, 2)}[kind]
+        dwh = torch.empty((3, *shape), device=device, dtype=torch.float32)
+        dbi = torch.empty((3, H), device=device, dtype=torch.float32) if want_bi else None
+        dbh = torch.empty((3, H), device=device, dtype=torch.float32)
+        scratch = torch.empty(scratch_bytes, device=device, dtype=torch.uint8)
+        ptrs = _BWD_PTRS(x.data_ptr(), h0.data_ptr(), out.data_ptr(), dout.data_ptr(), save.data_ptr(), kept.data_ptr(),
+                         scratch.data_ptr(), dx.data_ptr() if want_dx else None, dh0.data_ptr(),
+                         dwi.data_ptr() if want_wi else None, dwh.data_ptr(), dbi.data_ptr() if want_bi else None, dbh.data_ptr())
+        rc = _call(_lib.load().b200gru_layer_backward, dims, ctx.quants, ptrs, device)
+        if rc:
+            _lib._raise(rc, f"{kind} layer backward")
+        _lib._after_call()
+        none = (None, None, None)
+        grads = [dx, dh0, None, None, *(dwi.unbind(0) if want_wi else none), *dwh.unbind(0)]
+        if has_bias:
+            grads += [*(dbi.unbind(0) if want_bi else none), *dbh.unbind(0)]
+        return tuple(g if n else None for g, n in zip(grads, need))
+
+
+def forward(layer, x, h0):
+    """``out[T,B,H]``, or None where this path does not take the call."""
+    from .gru_layer import _extract_h_quant_params
+    cell, kind = layer.cell, layer._dispatch_kind
+    I, H = cell.input_size, cell.hidden_size
+    device = x.device
+    if (not cell._input_dense or I % 8 or H % 8 or not _plain_input(x, device) or not _plain_input(h0, device) or
+            x.shape[2] != I or h0.dim() != 2 or h0.shape[0] != x.shape[1] or h0.shape[1] != H or _transformed()):
+        return None
+    mods = cell._modules
+    bits_i = _weight_bits([mods["quant_W_i" + g] for g in _GATES])
+    bits_h = _weight_bits([mods["quant_W_h" + g] for g in _GATES]) if kind == "dense" else 32
+    if bits_i is None or bits_h is None:
+        return None
+    found = _parameters(cell, kind, device, I, H)
+    if found is None:
+        return None
+    params, nblocks, log2_hpad = found
+    grad = torch.is_grad_enabled() and (x.requires_grad or h0.requires_grad or any([p.requires_grad for p in params]))
+    qx = None
+    quant_x = mods["quant_x"]
+    if type(quant_x) is not Identity:
+        qx = None if grad else _extract_h_quant_params(quant_x)
+        if qx is None or qx[1] < -127 or qx[2] > 127:
+            qx, x = None, quant_x(x)
+            if not _plain_input(x, device):
+                return None
+    x, h0 = x.contiguous(), h0.contiguous()
+    if x.data_ptr() & 15:
+        return None
+    T, B = x.shape[0], x.shape[1]
+    key = (kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h)
+    if _plan(*key, _TRAIN if grad else 0) is None:
+        return None
+    quants = _quants(qx, _extract_h_quant_params(mods["quant_h_in"]), _extract_h_quant_params(mods["quant_h_out"]))
+    if grad:
+        return LayerFunction.apply(x, h0, key, quants, *params)
+    return _run(x, h0, key + (0,), quants, params, False)[0]
+
+
+def _plain_input(t, device):
+    return type(t) is torch.Tensor and t.dtype is torch.float32 and t.is_cuda and t.device == device

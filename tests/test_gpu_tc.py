@@ -328,3 +328,97 @@ def test_zz_bounded_wait_gives_up_and_is_reported():
     a = torch.randint(-127, 128, (128, 128), device="cuda", dtype=torch.int8)
     assert torch.equal(tc.gemm(a, a).cpu().double(), a.cpu().double() @ a.cpu().double().T)
     _lib.check_device_status()
+
+
+# ---- layer calls through one library entry -------------------------------------------------------------
+
+_LAYER_FORMS = [
+    ("dense", {}), ("dense", dict(wbits=8, hbits=8)), ("dense", dict(wbits=8, hbits=8, xbits=8)), ("dense", dict(wbits=4)),
+    ("dense", dict(xbits=8)), ("dense", dict(bias=False)), ("dense", dict(batch_first=True)), ("dense", dict(strided=True)),
+    ("dense", dict(frozen="i")), ("dense", dict(frozen="h")), ("diagonal", {}), ("diagonal", dict(hbits=8, T=40, B=70)),
+    ("monarch", dict(hbits=8)), ("butterfly", {}), ("butterfly", dict(H=24, bias=False)), ("dense", dict(flat=True)),
+]
+
+
+@pytest.mark.parametrize("kind,form", _LAYER_FORMS, ids=lambda v: v if isinstance(v, str) else "-".join(v) or "plain")
+@pytest.mark.parametrize("grad", [False, True], ids=["infer", "train"])
+def test_layer_entry_matches_the_composed_path(kind, form, grad, monkeypatch):
+    """``layer_native.forward`` against the same layer through ``tc.linear`` and the scan functions, over the forms
+    both accept.  Both split fp32 operands to 2^-22 of a term or better; states on a grid may part by one code where a
+    sum falls next to a half-way point, so those compare in norm."""
+    import gru_triton_b200 as gru
+    from gru_triton_b200 import layer_native
+    from gru_triton_b200.gru_cell import GRUCellQuant
+    T, B, I, H = form.get("T", 7), form.get("B", 5), 40, form.get("H", 64)
+    recipe = gru.QuantRecipe(weight=gru.QuantizerConfig(bits=form.get("wbits", 32), axis=0),
+                             input_act=gru.QuantizerConfig(bits=form.get("xbits", 32)),
+                             hidden=gru.QuantizerConfig(bits=form.get("hbits", 32)))
+    struct = None if kind == "dense" else gru.StructureConfig(kind=kind, nblocks=4, butterfly_nblocks=2)
+    torch.manual_seed(3)
+    layer = gru.GRULayer(I, H, recipe, gate_layout="fused", structure_hidden=struct, batch_first=form.get("batch_first", False))
+    if form.get("bias") is False:
+        layer.cell = GRUCellQuant(I, H, recipe, gate_layout="fused", bias=False, structure_hidden=struct)
+    layer = layer.cuda()
+    cell = layer.cell
+    if form.get("flat"):                       # parameters as views into one buffer, at addresses no vector load may use
+        flat = torch.empty(sum(p.numel() + 1 for p in layer.parameters()) + 1, device="cuda")
+        at = 1
+        for p in layer.parameters():
+            flat[at:at + p.numel()].copy_(p.detach().reshape(-1))
+            p.data = flat[at:at + p.numel()].view(p.shape)
+            at += p.numel() + 1
+    for q, s in ((cell.quant_x, 0.03), (cell.quant_h_in, 1 / 127.0), (cell.quant_h_out, 1 / 127.0)):
+        q.scale = torch.tensor(s, device="cuda")
+        q.freeze()
+    for name, p in layer.named_parameters():
+        if form.get("frozen") and f"_{form['frozen']}" in name.split(".")[-1]:
+            p.requires_grad_(False)
+    x = torch.randn(T, B, I, device="cuda")
+    if form.get("batch_first"):
+        x = x.transpose(0, 1).contiguous()
+    if form.get("strided"):
+        x = torch.randn(T, B, 2 * I, device="cuda")[..., ::2]
+    h0 = torch.randn(B, H, device="cuda") * 0.1
+    results = []
+    for native in (True, False):
+        taken = []
+        if native:
+            inner = layer_native.forward
+            monkeypatch.setattr(layer_native, "forward", lambda *a: taken.append(inner(*a)) or taken[-1])
+        else:
+            monkeypatch.setattr(layer_native, "forward", lambda *a: None)
+        layer.zero_grad(set_to_none=True)
+        xg, hg = x.detach().requires_grad_(grad), h0.detach().requires_grad_(grad)
+        with torch.set_grad_enabled(grad):
+            out, h_T = layer(xg, hg)
+        got = [out, h_T]
+        if grad:
+            torch.manual_seed(9)
+            out.backward(torch.randn_like(out))
+            got += [xg.grad, hg.grad] + [p.grad for p in layer.parameters()]
+        assert native is False or taken[0] is not None
+        monkeypatch.undo()
+        results.append(got)
+    tol = 1e-2 if form.get("hbits", 32) < 32 else 2e-5
+    for a, b in zip(*results):
+        assert (a is None) == (b is None)
+        if a is not None:
+            assert a.shape == b.shape and float((a - b).detach().norm()) <= tol * float(b.detach().norm()) + 1e-12
+
+
+def test_layer_entry_leaves_other_forms_to_the_composed_path():
+    import gru_triton_b200 as gru
+    from gru_triton_b200 import layer_native
+    off = gru.QuantizerConfig(bits=32, axis=0)
+    fp32 = gru.QuantRecipe(weight=off, input_act=off, hidden=off)
+    layer = gru.GRULayer(40, 64, fp32, gate_layout="fused").cuda()
+    h0 = torch.zeros(3, 64, device="cuda")
+    x = torch.randn(2, 3, 40, device="cuda")
+    assert layer_native.forward(layer, x, h0) is not None
+    assert layer_native.forward(layer, x.double(), h0.double()) is None
+    assert layer_native.forward(layer, x, h0[:2]) is None
+    assert layer_native.forward(layer, x[..., :32], h0) is None
+    with torch.autograd.forward_ad.dual_level():
+        assert layer_native.forward(layer, x, h0) is None
+    odd = gru.GRULayer(41, 64, fp32, gate_layout="fused").cuda()
+    assert layer_native.forward(odd, torch.randn(2, 3, 41, device="cuda"), h0) is None
