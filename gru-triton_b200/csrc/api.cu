@@ -26,9 +26,9 @@ int diag_backward(const float* gi, const float* h0, const float* W, const float*
                   int B, int H, Quant qi, Quant qo, cudaStream_t st);
 
 static std::atomic<unsigned long long> g_launches{0};
-static std::atomic<int> g_test_choice[3] = {{0}, {0}, {0}};
+static std::atomic<int> g_test_choice[4] = {{0}, {0}, {0}, {0}};
 
-int test_kernel_choice(int slot) { return (slot >= 0 && slot < 3) ? g_test_choice[slot].load(std::memory_order_relaxed) : 0; }
+int test_kernel_choice(int slot) { return (slot >= 0 && slot < 4) ? g_test_choice[slot].load(std::memory_order_relaxed) : 0; }
 static thread_local char g_last_error[256] = {0};
 
 void note_launch(int n) { g_launches.fetch_add((unsigned long long)n, std::memory_order_relaxed); }
@@ -585,6 +585,8 @@ int b200gru_dense_q8_backward(const float* gi, const float* h0, const float* Wq,
 }
 
 void b200gru_test_select_dense_scan(int which) { g_test_choice[2].store(which, std::memory_order_relaxed); }
+
+void b200gru_test_select_gemm(int which) { g_test_choice[3].store(which, std::memory_order_relaxed); }
 
 void b200gru_test_select_kernels(int butterfly_register_kernels, int diagonal_register_ring) {
   g_test_choice[0].store(butterfly_register_kernels, std::memory_order_relaxed);

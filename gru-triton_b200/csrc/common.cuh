@@ -175,12 +175,13 @@ int bfly_read_status(int reset);     // same for the staged butterfly kernels (b
 namespace tc {
 int tc_read_status(int reset);       // tensor-core GEMM core (tc_gemm.cu)
 int tc_step_read_status(int reset);  // fused tensor-core step (tc_step.cu)
+int tc2_read_status(int reset);      // CTA-pair products (tc_gemm2.cu)
 }  // namespace tc
 
 // Test hook (b200gru_test_select_kernels): slot 0 != 0 -> butterfly launches use the register /
 // global-twiddle kernels on every shape; slot 1 != 0 -> the diagonal forward uses the register-ring
 // kernel on every shape.  Slot 2 (b200gru_test_select_dense_scan): 1 -> FP32 cluster kernels, 2 -> tensor-core
-// cluster scan wherever it applies.  Defaults 0: the dispatch is by shape only.
+// cluster scan wherever it applies.  Slot 3 (b200gru_test_select_gemm): 1 -> single CTAs, 2 -> CTA pairs.  Defaults 0: the dispatch is by shape only.
 int test_kernel_choice(int slot);
 
 // Launch bookkeeping shared by all translation units (defined in api.cu).

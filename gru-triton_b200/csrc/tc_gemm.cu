@@ -558,6 +558,19 @@ int tc_gemm_tile_n(const TcGemm& g) {
   return best;
 }
 
+// CTA pairs take 256 x 256 tiles.  Measured single CTAs -> pairs with at least 48 such tiles: M = 32768, N = 3072, K = 1024,
+// three products 565 -> 486 us (1096 -> 1273 TFLOP/s), K = 512 269 -> 213 us at M = 24000; gradient 3072 x 1024 over 8192 rows
+// 131 -> 120 us; 48 tiles of K = 512 24.1 -> 23.4 us.  With fewer tiles narrower ones spread over more SMs.
+static bool pairs_apply(const TcGemm& g) {
+  const int which = test_kernel_choice(3);
+  if (which == 1) return false;
+  const int splits = g.split_k < 1 ? 1 : g.split_k;
+  if (cdiv(cdiv(g.K, tc_gemm_kblock(g)), cdiv(cdiv(g.K, tc_gemm_kblock(g)), splits)) != splits) return false;
+  if (which == 2) return true;
+  if (g.tile_n != 0 && g.tile_n != 256) return false;
+  return g.M > 128 && g.N > 128 && (long long)cdiv(g.M, 256) * cdiv(g.N, 256) * splits >= 48;
+}
+
 int launch_tc_gemm(const TcGemm& g, cudaStream_t st) {
   const bool i8 = g.kind == TC_KIND_I8;
   const int es = i8 ? 1 : 2;
@@ -570,6 +583,10 @@ int launch_tc_gemm(const TcGemm& g, cudaStream_t st) {
   if ((g.N & 3) || (g.ldc & 3) || !aligned16(g.C) || !aligned16(g.A) || !aligned16(g.B)) return B200GRU_INVALID_ARGUMENT;
   if (((g.lda * es) & 15) || ((g.ldb * es) & 15) || ((g.a_plane_stride * es) & 15) || ((g.b_plane_stride * es) & 15))
     return B200GRU_INVALID_ARGUMENT;
+  if (pairs_apply(g)) {
+    const int rc = launch_tc_gemm_pairs(g, st);
+    if (rc != B200GRU_UNSUPPORTED) return rc;
+  }
   const int bn = tc_gemm_tile_n(g);
   if (bn == 0) return B200GRU_UNSUPPORTED;
   const int ke = 128 / es;

@@ -47,6 +47,8 @@ int tc_gemm_kblock(const TcGemm& g);
 int tc_gemm_splits(const TcGemm& g, int want);
 int tc_gemm_tile_n(const TcGemm& g);
 int launch_tc_gemm(const TcGemm& g, cudaStream_t st);
+// The same by persistent CTA pairs (tc_gemm2.cu); launch_tc_gemm() checks the arguments and chooses.
+int launch_tc_gemm_pairs(const TcGemm& g, cudaStream_t st);
 
 // Launches the bounded-wait probe (a wait that must run out); sets the tensor-core health word.
 int launch_wait_timeout_probe(cudaStream_t st);

@@ -326,11 +326,14 @@ int b200gru_calibration_scan(const b200gru_shape* shape, const float* gi, const 
  * tests can hold both to the same parity bar.  Process-wide; (0, 0) restores the normal dispatch.
  * b200gru_test_select_dense_scan: 1 makes dense / block-diagonal scans use the FP32 cluster kernels,
  * 2 the tensor-core cluster scan wherever it applies; 0 restores the choice by shape.
+ * b200gru_test_select_gemm: 1 makes the tensor-core products use single CTAs, 2 pairs of CTAs; 0 the
+ * choice by shape.
  * b200gru_test_wait_timeout: launches one tiny kernel whose bounded wait must run out (it waits
  * about a millisecond for bytes nothing sends), which sets the flag b200gru_device_status
  * reports; the kernel returns normally and the device stays usable. */
 void b200gru_test_select_kernels(int butterfly_register_kernels, int diagonal_register_ring);
 void b200gru_test_select_dense_scan(int which);
+void b200gru_test_select_gemm(int which);
 int b200gru_test_wait_timeout(void* stream);
 
 /* Human-readable text for a b200gru_status; plus the text of the last CUDA error

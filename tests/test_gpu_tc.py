@@ -330,6 +330,38 @@ def test_zz_bounded_wait_gives_up_and_is_reported():
     _lib.check_device_status()
 
 
+@pytest.mark.parametrize("dtype,M,N,K,pa,pb,a_mn,b_mn,split", [
+    ("f16", 256, 256, 64, 1, 1, False, False, 1), ("f16", 300, 520, 200, 2, 2, False, False, 1),
+    ("bf16", 136, 264, 1024, 2, 2, True, True, 1), ("bf16", 513, 304, 520, 3, 3, False, True, 1),
+    ("bf16", 520, 304, 776, 2, 1, True, False, 1), ("i8", 300, 512, 1040, 1, 1, False, False, 1),
+    ("bf16", 1536, 512, 2048, 2, 2, True, True, 4), ("f16", 40000, 260, 96, 2, 2, False, False, 1)])
+def test_cta_pair_products_equal_single_cta_products(dtype, M, N, K, pa, pb, a_mn, b_mn, split):
+    """Both kernels add the same products in the same order, so the results are the same bits: edges of the 256 x 256
+    tiles, one tile and more than the device has pairs, K slices, every operand layout."""
+    from gru_triton_b200 import _lib
+    tc = _tc()
+    torch.manual_seed(M + N + K)
+    def operand(planes, rows, mn):
+        shape = (planes, K, rows) if mn else (planes, rows, K)
+        if dtype == "i8":
+            return torch.randint(-127, 128, shape, device="cuda", dtype=torch.int8)
+        return torch.randn(shape, device="cuda").to(torch.float16 if dtype == "f16" else torch.bfloat16)
+    A, B = operand(pa, M, a_mn), operand(pb, N, b_mn)
+    pairs = [(i, j) for s in range(3) for i in range(s + 1) for j in [s - i] if i < pa and j < pb]
+    bias, rs, cs = torch.randn(N, device="cuda"), torch.rand(M, device="cuda"), torch.rand(N, device="cuda")
+    results = []
+    for which in (1, 2):
+        _lib.load().b200gru_test_select_gemm(which)
+        try:
+            out = torch.ones(M, N, device="cuda") if split == 1 else None
+            results.append(tc.gemm(A, B, a_mn=a_mn, b_mn=b_mn, pairs=pairs, split_k=split, row_scale=rs, col_scale=cs, bias=bias,
+                                   out=out, accumulate=split == 1, tile_n=256 if pa + pb < 6 else 0).clone())
+            torch.cuda.synchronize()
+        finally:
+            _lib.load().b200gru_test_select_gemm(0)
+    assert torch.equal(*results)
+
+
 # ---- layer calls through one library entry -------------------------------------------------------------
 
 _LAYER_FORMS = [
