@@ -119,7 +119,9 @@ void launch_reduce_partials(const float* src, int nparts, size_t row_stride, siz
   }
   // one thread per column group already fills the chip above 2^17 groups; below that the partials are spread
   const size_t groups = n / 4;
-  if (nparts >= 16 && groups < ((size_t)1 << 14))
+  if (nparts >= 4 && nparts < 16 && groups < ((size_t)1 << 14))
+    launch_pdl(reduce_partials4_kernel<4>, dim3((unsigned)((groups + 63) / 64)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
+  else if (nparts >= 16 && groups < ((size_t)1 << 14))
     launch_pdl(reduce_partials4_kernel<8>, dim3((unsigned)((groups + 31) / 32)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
   else
     launch_pdl(reduce_partials4_kernel<1>, dim3((unsigned)((groups + 255) / 256)), dim3(256), 0, st, src, nparts, row_stride, n, dst);

@@ -998,13 +998,14 @@ bool choose_block_config(bool fwd, int T, int B, int Hb, int nb, BlockScanConfig
         const double wstream = 3.0 * Hc4 * Hb * 4.0 / (ws ? 128.0 : 24.0), hstream = (double)Hb * BT * 4.0 * NW / 128.0;
         double step;
         if (fwd) {
-          step = 0.6 * wstream + fma + hstream + (200.0 + 290.0 * BT) * ipw + (C > 1 ? 700.0 + 40.0 * C : 1000.0);
+          step = 0.6 * wstream + fma + hstream + (200.0 + 290.0 * BT) * ipw + (C > 1 ? 700.0 + 40.0 * C : (ipw > 1 ? 1000.0 : 700.0));
         } else {
-          const double barrier = C > 1 ? 1200.0 + 40.0 * C : 1400.0;
+          const double barrier = C > 1 ? 1200.0 + 40.0 * C : 1200.0;
           step = (fma > wstream + hstream ? fma : wstream + hstream) + barrier + 400.0;
           step += c.TW == 1 ? 45.0 * Hc4 * (BT - 1) / c.NH : 0.11 * (BT - 1) * step;
         }
-        const double cost = waves * (step + 25000.0 / T);
+        const double setup = fwd ? 8000.0 + 1100.0 * C : 11500.0 + 530.0 * C;       // launch, weight slice
+        const double cost = waves * (step + setup / T);
         if (cost < best) { best = cost; found = true; *out = c; }
         break;                                          // weights in smem fit: do not also try global
       }

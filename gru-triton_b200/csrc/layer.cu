@@ -358,10 +358,7 @@ int linear_backward(const Layer& L, const Kept& k, const float* x, const float* 
   return rc;
 }
 
-enum { FLAG_TRAIN = 1, FLAG_DX = 2, FLAG_DWI = 4, FLAG_DBI = 8 };
-
 size_t scan_ws(const Layer& L, int backward) { return pad(b200gru_workspace_bytes(&L.shape, backward)); }
-size_t gi_bytes(const Layer& L) { return pad(L.rows * 3 * L.H * 4); }
 bool keeps_gi(const Layer& L) { return L.shape.kind == B200GRU_DIAGONAL; }     // recomputes its gates instead of saving them
 
 b200gru_quant quant_of(const float* q) {
@@ -382,13 +379,12 @@ int b200gru_layer_sizes(const int* dims, size_t* sizes) {
   Kept k;
   if (!parse(dims, &L)) return B200GRU_INVALID_ARGUMENT;
   if (b200gru_workspace_bytes(&L.shape, 0) == (size_t)-1) return B200GRU_UNSUPPORTED;
-  const bool train = (L.flags & FLAG_TRAIN) != 0;
   const int mode = keeps_gi(L) ? 1 : 2;
   sizes[0] = carve(L, nullptr, &k);
   const size_t fwd_scan = scan_ws(L, 0), proj = x_planes_bytes(L);
-  sizes[1] = (fwd_scan > proj ? fwd_scan : proj) + (train && keeps_gi(L) ? 0 : gi_bytes(L));
+  sizes[1] = fwd_scan > proj ? fwd_scan : proj;
   const size_t bwd_scan = scan_ws(L, mode), lin = linear_plan(L).total;
-  sizes[2] = (bwd_scan > lin ? bwd_scan : lin) + gi_bytes(L) + (L.bits_h <= 8 ? pad(L.w_elems * 4) : 0);
+  sizes[2] = (bwd_scan > lin ? bwd_scan : lin) + (L.bits_h <= 8 ? pad(L.w_elems * 4) : 0);
   return B200GRU_OK;
 }
 
@@ -402,8 +398,9 @@ int b200gru_layer_forward(const int* dims, const float* quants, const void* cons
   float* out = static_cast<float*>(const_cast<void*>(ptrs[14]));
   float* save = static_cast<float*>(const_cast<void*>(ptrs[15]));
   char* kept = static_cast<char*>(const_cast<void*>(ptrs[16]));
-  char* scratch = static_cast<char*>(const_cast<void*>(ptrs[17]));
-  if (!x || !h0 || !out || !kept || !scratch) return B200GRU_INVALID_ARGUMENT;
+  char* ws = static_cast<char*>(const_cast<void*>(ptrs[17]));
+  float* gi = static_cast<float*>(const_cast<void*>(ptrs[18]));
+  if (!x || !h0 || !out || !kept || !ws || !gi) return B200GRU_INVALID_ARGUMENT;
   for (int i = 0; i < 6; ++i) if (p[i] == nullptr) return B200GRU_INVALID_ARGUMENT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   carve(L, kept, &k);
@@ -412,15 +409,10 @@ int b200gru_layer_forward(const int* dims, const float* quants, const void* cons
     return B200GRU_INVALID_ARGUMENT;
   int rc = gather_weights(L, k, p, p + 3, p + 6, p + 9, st);
   if (rc) return rc;
-  // the diagonal backward recomputes its gates from gi: a training step keeps it (in the place of `save`)
-  const bool gi_out = (L.flags & FLAG_TRAIN) && keeps_gi(L);
-  float* gi = gi_out ? save : reinterpret_cast<float*>(scratch);
-  char* ws = gi_out ? scratch : scratch + gi_bytes(L);
-  if (gi == nullptr) return B200GRU_INVALID_ARGUMENT;
   rc = project(L, k, x, make_quant(&qx), gi, ws, st);
   if (rc) return rc;
   const size_t n = scan_ws(L, 0);
-  float* S = gi_out ? nullptr : save;
+  float* S = keeps_gi(L) ? nullptr : save;
   if (L.bits_h <= 8)
     return b200gru_dense_q8_forward(gi, h0, k.Wh_q, k.Wh_codes, k.Wh_scale, k.b_h, L.T, L.B, L.H, &qi, &qo, out, S, ws, n, stream);
   return b200gru_scan_forward(&L.shape, gi, h0, k.Wh, k.b_h, &qi, &qo, out, S, ws, n, stream);
@@ -437,12 +429,12 @@ int b200gru_layer_backward(const int* dims, const float* quants, const void* con
   const float* save = static_cast<const float*>(ptrs[4]);
   char* kept = static_cast<char*>(const_cast<void*>(ptrs[5]));
   char* scratch = static_cast<char*>(const_cast<void*>(ptrs[6]));
-  float* const* o = reinterpret_cast<float* const*>(const_cast<void* const*>(ptrs)) + 7;   // dx, dh0, dWi, dWh, dbi, dbh
-  if (!x || !h0 || !out || !dout || !save || !kept || !scratch || !o[1] || !o[3] || !o[5]) return B200GRU_INVALID_ARGUMENT;
+  float* const* o = reinterpret_cast<float* const*>(const_cast<void* const*>(ptrs)) + 7;   // dx, dh0, dWi, dWh, dbi, dbh, dgi
+  if (!x || !h0 || !out || !dout || !save || !kept || !scratch || !o[1] || !o[3] || !o[5] || !o[6]) return B200GRU_INVALID_ARGUMENT;
   carve(L, kept, &k);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const b200gru_quant qi = quant_of(quants + 4), qo = quant_of(quants + 8);
-  float* dgi = reinterpret_cast<float*>(scratch); scratch += gi_bytes(L);
+  float* dgi = o[6];
   float* dWq = nullptr;
   if (L.bits_h <= 8) { dWq = reinterpret_cast<float*>(scratch); scratch += pad(L.w_elems * 4); }
   int rc;                               // gi is read only where the gates were not saved; dgi stands in for it

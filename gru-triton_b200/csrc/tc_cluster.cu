@@ -589,11 +589,12 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
       const bool own = u0 + j < Hb;
       float s = 1.f, inv = 1.f;
       if (PW == 2) {
+        // All loads in flight at once, from clamped addresses (an entry read twice does not change the maximum): under a
+        // condition each waited for the one before it, and the prologue took 28 us at H = 512 instead of 17.
+        const float* src = a.W + (size_t)g * a.w_gate_stride + (size_t)n * a.w_block_stride + (size_t)(own ? u0 + j : 0) * Hb;
         float mx = 0.f;
-        if (own) {
-          const float* src = a.W + (size_t)g * a.w_gate_stride + (size_t)n * a.w_block_stride + (size_t)(u0 + j) * Hb;
-          for (int k = lane; k < Hb; k += 32) mx = fmaxf(mx, fabsf(__ldg(src + k)));
-        }
+#pragma unroll
+        for (int q = 0; q < TILES * 4; ++q) mx = fmaxf(mx, fabsf(__ldg(src + min(lane + 32 * q, Hb - 1))));
         pow2_row_scale(warp_max(mx), &s, &inv);
       } else {
         inv = own ? a.scales[g * H + u0 + j] : 0.f;
@@ -614,19 +615,21 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
 #pragma unroll 1
     for (int g = 0; g < 3; ++g) {
       uint32_t vh[16], vl[16];
+      const int kc = min(k, Hb - 1);
+      float w[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int jr = min(u0 + j, Hb - 1);
+        w[j] = PW == 1 ? (float)a.codes[((size_t)g * H + jr) * Hb + kc]
+                       : __ldg(a.W + (size_t)g * a.w_gate_stride + (size_t)n * a.w_block_stride + (size_t)jr * Hb + kc);
+      }
 #pragma unroll
       for (int j2 = 0; j2 < 16; ++j2) {
         __half hi[2], lw[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int j = 2 * j2 + e;
-          float v = 0.f;
-          if (k < Hb && u0 + j < Hb) {
-            if (PW == 1) v = (float)a.codes[((size_t)g * H + u0 + j) * Hb + k];
-            else v = __ldg(a.W + (size_t)g * a.w_gate_stride + (size_t)n * a.w_block_stride + (size_t)(u0 + j) * Hb + k) *
-                     s_scale[g * 32 + j];
-          }
-          split2(v, &hi[e], &lw[e]);
+          split2((k < Hb && u0 + j < Hb) ? w[j] * s_scale[g * 32 + j] : 0.f, &hi[e], &lw[e]);
         }
         vh[j2] = pack2(hi[0], hi[1]);
         vl[j2] = pack2(lw[0], lw[1]);
@@ -953,7 +956,9 @@ bool choose(bool fwd, int T, int B, int Hb, int nb, bool w_codes, const Quant& q
     const double slab = fwd ? (double)ph * ((rows + 7) / 8 * 8) * 64 : (double)((rows + 3) / 4) * 512;
     const double step = fwd ? 750.0 + C * (60.0 + slab / 15.0) + 1000.0 * (N / 16)
                             : 1300.0 + C * (50.0 + slab / 8.3) + 1000.0 * (N / 16);
-    const double cost = waves * (step * T + 27000.0);
+    // set-up (weights into tensor memory), from T = 1 and T = 4 launches
+    const double setup = fwd ? 12000.0 + 750.0 * C : 18500.0 + 850.0 * C;
+    const double cost = waves * (step * T + setup);
     if (!found || cost < *cycles) {
       found = true;
       *cycles = cost;

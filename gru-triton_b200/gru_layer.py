@@ -19,6 +19,7 @@ from typing import Iterable, Optional
 import torch
 import torch.nn as nn
 
+from . import layer_native
 from .gru_cell import GateLayout, GRUCellQuant
 from .quantizers import FakeQuantize, FakeQuantizePerChannel, FakeQuantizePerTensor, Identity, QuantRecipe
 from .structure import StructureConfig
@@ -206,8 +207,7 @@ class GRULayer(nn.Module):
         """Input projection hoisted to one GEMM, then the persistent CUDA scan
         (gru_layer.py:234-302); one library call where the layer has the common form."""
         cell = self.cell
-        from . import layer_native
-        out = layer_native.forward(self, x, h0)
+        out = layer_native.forward(self, x, h0) if cell.input_size % 8 == 0 and self.hidden_size % 8 == 0 else None
         if out is not None:
             return (out.transpose(0, 1) if self.batch_first else out), out[-1]
         if cell._input_dense:

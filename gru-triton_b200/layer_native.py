@@ -20,19 +20,18 @@ import torch
 from . import _lib
 from .quantizers import FakeQuantizePerChannel, Identity
 
-_TRAIN, _DX, _DWI, _DBI = 1, 2, 4, 8
 _INTS = ctypes.c_int * 10
 _FLOATS = ctypes.c_float * 12
-_FWD_PTRS = ctypes.c_void_p * 18
-_BWD_PTRS = ctypes.c_void_p * 13
+_FWD_PTRS = ctypes.c_void_p * 19
+_BWD_PTRS = ctypes.c_void_p * 14
 _SIZES = ctypes.c_size_t * 3
 _GATES = "rzn"
 
 
 @lru_cache(maxsize=512)
-def _plan(kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h, flags):
+def _plan(kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h):
     """``(dims, kept bytes, forward scratch, backward scratch)`` of a shape, or None if it has none."""
-    dims = _INTS(_lib.KIND[kind], T, B, I, H, nblocks, log2_hpad, bits_i, bits_h, flags)
+    dims = _INTS(_lib.KIND[kind], T, B, I, H, nblocks, log2_hpad, bits_i, bits_h, 0)
     sizes = _SIZES()
     if _lib.load().b200gru_layer_sizes(dims, sizes):
         return None
@@ -119,18 +118,18 @@ def _run(x, h0, key, quants, params, train):
     kind, T, B, I, H = key[:5]
     device = x.device
     out = torch.empty((T, B, H), device=device, dtype=torch.float32)
-    save = None
-    if train:
-        save = torch.empty((T, B, 3 * H) if kind == "diagonal" else (4, T, B, H), device=device, dtype=torch.float32)
+    # the diagonal backward recomputes its gates from gi, the others read them
+    save = torch.empty((4, T, B, H), device=device, dtype=torch.float32) if train and kind != "diagonal" else None
     kept = torch.empty(kept_bytes, device=device, dtype=torch.uint8)
+    gi = torch.empty((T, B, 3 * H), device=device, dtype=torch.float32)
     scratch = torch.empty(scratch_bytes, device=device, dtype=torch.uint8)
     ptrs = _FWD_PTRS(x.data_ptr(), h0.data_ptr(), *_addresses(params), out.data_ptr(), None if save is None else save.data_ptr(),
-                     kept.data_ptr(), scratch.data_ptr())
+                     kept.data_ptr(), scratch.data_ptr(), gi.data_ptr())
     rc = _call(_lib.load().b200gru_layer_forward, dims, quants, ptrs, device)
     if rc:
         _lib._raise(rc, f"{kind} layer forward")
     _lib._after_call()
-    return out, save, kept
+    return out, (gi if kind == "diagonal" else save), kept
 
 
 def _call(fn, dims, quants, ptrs, device):
@@ -147,7 +146,7 @@ class LayerFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, h0, key, quants, *params):
         train = any(ctx.needs_input_grad)
-        out, save, kept = _run(x, h0, key[:9] + (_TRAIN if train else 0,), quants, params, train)
+        out, save, kept = _run(x, h0, key, quants, params, train)
         ctx.key, ctx.quants, ctx.nparams = key, quants, len(params)
         if train:
             ctx.save_for_backward(x, h0, out, save, kept)
@@ -160,7 +159,7 @@ class LayerFunction(torch.autograd.Function):
         kind, T, B, I, H, nblocks, log2_hpad = ctx.key[:7]
         has_bias = ctx.nparams == 12
         want_dx, want_wi, want_bi = need[0], any(need[4:7]), has_bias and any(need[10:13])
-        dims, _, _, scratch_bytes = _plan(*ctx.key[:9], _TRAIN)
+        dims, _, _, scratch_bytes = _plan(*ctx.key)
         device = x.device
         dout = dout.contiguous()
         dx = torch.empty_like(x) if want_dx else None
@@ -171,10 +170,11 @@ class LayerFunction(torch.autograd.Function):
         dwh = torch.empty((3, *shape), device=device, dtype=torch.float32)
         dbi = torch.empty((3, H), device=device, dtype=torch.float32) if want_bi else None
         dbh = torch.empty((3, H), device=device, dtype=torch.float32)
+        dgi = torch.empty((T, B, 3 * H), device=device, dtype=torch.float32)
         scratch = torch.empty(scratch_bytes, device=device, dtype=torch.uint8)
         ptrs = _BWD_PTRS(x.data_ptr(), h0.data_ptr(), out.data_ptr(), dout.data_ptr(), save.data_ptr(), kept.data_ptr(),
                          scratch.data_ptr(), dx.data_ptr() if want_dx else None, dh0.data_ptr(),
-                         dwi.data_ptr() if want_wi else None, dwh.data_ptr(), dbi.data_ptr() if want_bi else None, dbh.data_ptr())
+                         dwi.data_ptr() if want_wi else None, dwh.data_ptr(), dbi.data_ptr() if want_bi else None, dbh.data_ptr(), dgi.data_ptr())
         rc = _call(_lib.load().b200gru_layer_backward, dims, ctx.quants, ptrs, device)
         if rc:
             _lib._raise(rc, f"{kind} layer backward")
@@ -218,12 +218,12 @@ def forward(layer, x, h0):
         return None
     T, B = x.shape[0], x.shape[1]
     key = (kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h)
-    if _plan(*key, _TRAIN if grad else 0) is None:
+    if _plan(*key) is None:
         return None
     quants = _quants(qx, _extract_h_quant_params(mods["quant_h_in"]), _extract_h_quant_params(mods["quant_h_out"]))
     if grad:
         return LayerFunction.apply(x, h0, key, quants, *params)
-    return _run(x, h0, key + (0,), quants, params, False)[0]
+    return _run(x, h0, key, quants, params, False)[0]
 
 
 def _plain_input(t, device):

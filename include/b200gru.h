@@ -257,12 +257,14 @@ int b200gru_column_sums(const float* src, size_t rows, int cols, float* dst, voi
  * Stands in for GRULayer._forward_fast_dispatch (src/gru_qat/gru_layer.py:234-302) and its autograd.
  *   dims   {kind, T, B, I, H, nblocks, log2_hpad, weight bits of the input side, of the hidden side (dense), flags};
  *          I and H multiples of 8; bits 32 (none) or 2..8 (per output row, symmetric, dynamic scale);
- *          flags: 1 = a backward call follows
+ *          0 (reserved)
  *   quants {scale, qmin, qmax, enabled} of the input, fq_in and fq_out (frozen); the input one only where no backward follows
  *   sizes  bytes of the buffers {kept, forward scratch, backward scratch}, 256-byte aligned
  *   forward ptrs   {x[T][B][I], h0[B][H], Wi r,z,n, Wh r,z,n, bi r,z,n, bh r,z,n (biases may be NULL), out[T][B][H],
- *                   save (flags & 1: [4][T][B][H], diagonal: [T][B][3H]; else NULL), kept, scratch}
- *   backward ptrs  {x, h0, out, dout, save, kept, scratch, dx or NULL, dh0, dWi[3H][I] or NULL, dWh, dbi[3H] or NULL, dbh[3H]}
+ *                   save ([4][T][B][H] where a backward call follows, else NULL; diagonal: NULL), kept, scratch,
+ *                   gi[T][B][3H] (scratch; a diagonal backward reads it)}
+ *   backward ptrs  {x, h0, out, dout, save (diagonal: gi), kept, scratch, dx or NULL, dh0, dWi[3H][I] or NULL, dWh,
+ *                   dbi[3H] or NULL, dbh[3H], dgi[T][B][3H] (scratch)}
  * Hidden weights per gate: [H][H], [H], [nblocks][H/nblocks][H/nblocks] or [nblocks][log2_hpad][2^log2_hpad / 2][2][2]. */
 int b200gru_layer_sizes(const int* dims, size_t* sizes);
 int b200gru_layer_forward(const int* dims, const float* quants, const void* const* ptrs, void* stream);
