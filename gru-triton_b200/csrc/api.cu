@@ -18,11 +18,11 @@
 namespace b200gru {
 
 // diag_scan.cu
-size_t diag_bwd_workspace_bytes(int T, int B, int H);
+size_t diag_bwd_workspace_bytes(int T, int B, int H, bool input_bias);
 int diag_forward(const float* gi, const float* h0, const float* W, const float* bh, float* out, int T, int B,
                  int H, Quant qi, Quant qo, cudaStream_t st);
 int diag_backward(const float* gi, const float* h0, const float* W, const float* bh, const float* out,
-                  const float* dout, float* dgi, float* dh0, float* dW, float* dbh, void* workspace, int T,
+                  const float* dout, float* dgi, float* dh0, float* dW, float* dbh, float* dbi, void* workspace, int T,
                   int B, int H, Quant qi, Quant qo, cudaStream_t st);
 
 static std::atomic<unsigned long long> g_launches{0};
@@ -63,68 +63,80 @@ int allow_dynamic_smem(const void* kernel, size_t bytes) {
   return (it->second >= 0 && bytes <= (size_t)it->second) ? B200GRU_OK : B200GRU_UNSUPPORTED;
 }
 
-__global__ void reduce_partials_kernel(const float* __restrict__ src, int nparts, size_t row_stride, size_t n,
-                                       float* __restrict__ dst) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = src[i];
-  for (int p = 1; p < nparts; ++p) s += src[(size_t)p * row_stride + i];
-  dst[i] = s;
-}
+__device__ __forceinline__ void add_to(float& s, float v) { s += v; }
+__device__ __forceinline__ void add_to(float4& s, const float4& v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+__device__ __forceinline__ void set_zero(float& s) { s = 0.f; }
+__device__ __forceinline__ void set_zero(float4& s) { s = make_float4(0.f, 0.f, 0.f, 0.f); }
 
 // Sum of partial vectors, PY partial groups per block: thread (x, y) adds partials y, y + PY, ... of
-// four columns in order and the block adds the PY sums in order, so the result has a fixed order.
-// Memory latency bounds it: the one-thread-per-column loop before kept at most four 4-byte loads in
-// flight (64 partials of 1536 columns: 6 blocks, 18 us); here a column's partials are spread over
-// up to eight threads with up to eight 16-byte loads in flight each.
-template <int PY>
+// four columns (one where a pointer is not 16-byte aligned) in order and the block adds the PY sums in
+// order, so the result has a fixed order.  Memory latency bounds it: one thread per column with 4-byte
+// loads kept at most four of them in flight (64 partials of 1536 columns: 6 blocks, 18 us); here a
+// column's partials are spread over up to eight threads with up to eight loads in flight each.
+template <int PY, typename V>
 __global__ void __launch_bounds__(256)
-reduce_partials4_kernel(const float* __restrict__ src, int nparts, size_t row_stride, size_t n, float* __restrict__ dst) {
+reduce_partials_kernel(const V* __restrict__ src, int nparts, size_t row_stride, size_t n, const ReduceTargets t) {
   constexpr int PX = 256 / PY;
-  __shared__ float4 part[PY > 1 ? PY : 1][PX];
+  __shared__ V part[PY][PX];
   pdl_launch_dependents();
   pdl_wait();
   const int tx = threadIdx.x % PX, ty = threadIdx.x / PX;
-  const size_t i = ((size_t)blockIdx.x * PX + tx) * 4;
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  const size_t i = (size_t)blockIdx.x * PX + tx;
+  V s;
+  set_zero(s);
   if (i < n) {
 #pragma unroll 8
-    for (int p = ty; p < nparts; p += PY) {
-      const float4 v = __ldcs(reinterpret_cast<const float4*>(src + (size_t)p * row_stride + i));
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-    }
+    for (int p = ty; p < nparts; p += PY) add_to(s, __ldcs(src + (size_t)p * row_stride + i));
   }
   if (PY > 1) {
     part[ty][tx] = s;
     __syncthreads();
     if (ty != 0) return;
 #pragma unroll
-    for (int y = 1; y < PY; ++y) {
-      const float4 v = part[y][tx];
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    for (int y = 1; y < PY; ++y) add_to(s, part[y][tx]);
+  }
+  if (i >= n) return;
+  constexpr size_t E = sizeof(V) / sizeof(float);
+#pragma unroll
+  for (int k = 0; k < ReduceTargets::MAX; ++k) {
+    if (k >= t.count) break;
+    if (i * E >= t.begin[k] && i * E < t.end[k]) {
+      const size_t at = i * E - t.begin[k];
+      *reinterpret_cast<V*>(t.a[k] + at) = s;
+      if (t.b[k] != nullptr) *reinterpret_cast<V*>(t.b[k] + at) = s;
     }
   }
-  if (i < n) *reinterpret_cast<float4*>(dst + i) = s;
+}
+
+template <typename V>
+static void launch_reduce_typed(const float* src, int nparts, size_t row_stride, size_t n, const ReduceTargets& t, cudaStream_t st) {
+  constexpr size_t E = sizeof(V) / sizeof(float);
+  const V* s = reinterpret_cast<const V*>(src);
+  n /= E; row_stride /= E;
+  // one thread per column group fills the chip from 2^14 groups; below that the partials are spread
+  const int py = n >= ((size_t)1 << 14) || nparts < 4 ? 1 : (nparts < 16 ? 4 : 8);
+  const dim3 grid((unsigned)((n * py + 255) / 256));
+  if (py == 8) launch_pdl(reduce_partials_kernel<8, V>, grid, dim3(256), 0, st, s, nparts, row_stride, n, t);
+  else if (py == 4) launch_pdl(reduce_partials_kernel<4, V>, grid, dim3(256), 0, st, s, nparts, row_stride, n, t);
+  else launch_pdl(reduce_partials_kernel<1, V>, grid, dim3(256), 0, st, s, nparts, row_stride, n, t);
+  note_launch();
+}
+
+void launch_reduce_targets(const float* src, int nparts, size_t row_stride, size_t n, const ReduceTargets& t, cudaStream_t st) {
+  bool vec = n % 4 == 0 && row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+  for (int k = 0; k < t.count; ++k)
+    vec = vec && t.begin[k] % 4 == 0 && t.end[k] % 4 == 0 &&
+          ((reinterpret_cast<uintptr_t>(t.a[k]) | reinterpret_cast<uintptr_t>(t.b[k])) & 15u) == 0;
+  if (vec) launch_reduce_typed<float4>(src, nparts, row_stride, n, t, st);
+  else launch_reduce_typed<float>(src, nparts, row_stride, n, t, st);
 }
 
 void launch_reduce_partials(const float* src, int nparts, size_t row_stride, size_t n, float* dst,
                             cudaStream_t st) {
-  const bool vec = n % 4 == 0 && row_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
-  note_launch();
-  if (!vec) {
-    launch_pdl(reduce_partials_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
-    return;
-  }
-  // one thread per column group already fills the chip above 2^17 groups; below that the partials are spread
-  const size_t groups = n / 4;
-  if (nparts >= 4 && nparts < 16 && groups < ((size_t)1 << 14))
-    launch_pdl(reduce_partials4_kernel<4>, dim3((unsigned)((groups + 63) / 64)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
-  else if (nparts >= 16 && groups < ((size_t)1 << 14))
-    launch_pdl(reduce_partials4_kernel<8>, dim3((unsigned)((groups + 31) / 32)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
-  else
-    launch_pdl(reduce_partials4_kernel<1>, dim3((unsigned)((groups + 255) / 256)), dim3(256), 0, st, src, nparts, row_stride, n, dst);
+  ReduceTargets t;
+  memset(&t, 0, sizeof(t));
+  t.add(0, n, dst, nullptr);
+  launch_reduce_targets(src, nparts, row_stride, n, t, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -197,7 +209,7 @@ static size_t workspace_bytes(const Dims& d, int backward) {
                       tc::tc_weight_grads_scratch_bytes(d.T, d.B, d.H, true));
       return s_need + weight_grads_scratch_bytes(d.T, d.B, d.H, d.nb, d.Hb);
     case B200GRU_DIAGONAL:
-      return backward ? diag_bwd_workspace_bytes(d.T, d.B, d.H) : 0;
+      return backward ? diag_bwd_workspace_bytes(d.T, d.B, d.H, true) : 0;
     case B200GRU_BUTTERFLY: {
       const size_t twp = align_up(d.w_elems * sizeof(float), 256);      // twiddles in pass order
       if (!backward) return twp;
@@ -350,7 +362,7 @@ static int scan_backward_impl(const b200gru_shape* shape, const float* gi, const
                               const signed char* codes, const float* scales,
                               const float* bh, const float* out, const float* dout, const float* save,
                               const b200gru_quant* q_in, const b200gru_quant* q_out, float* dgi, float* dh0,
-                              float* dW, float* dbh, void* workspace, size_t workspace_bytes_, void* stream) {
+                              float* dW, float* dbh, float* dbi, void* workspace, size_t workspace_bytes_, void* stream) {
   Dims d;
   if (!parse_shape(shape, &d)) return B200GRU_INVALID_ARGUMENT;
   if (!gi || !h0 || !W || !bh || !out || !dout || !dgi || !dh0 || !dW || !dbh) return B200GRU_INVALID_ARGUMENT;
@@ -366,7 +378,7 @@ static int scan_backward_impl(const b200gru_shape* shape, const float* gi, const
 
   switch (d.kind) {
     case B200GRU_DIAGONAL:
-      return diag_backward(gi, h0, W, bh, out, dout, dgi, dh0, dW, dbh, workspace, d.T, d.B, d.H, qi, qo, st);
+      return diag_backward(gi, h0, W, bh, out, dout, dgi, dh0, dW, dbh, dbi, workspace, d.T, d.B, d.H, qi, qo, st);
     case B200GRU_DENSE:
     case B200GRU_MONARCH: {
       float* S_ws = reinterpret_cast<float*>(ws);
@@ -374,7 +386,7 @@ static int scan_backward_impl(const b200gru_shape* shape, const float* gi, const
       BlockGemmArgs g;
       memset(&g, 0, sizeof(g));
       g.gi = gi; g.h0 = h0; g.out = out; g.W = W; g.bh = bh; g.dgi = dgi;
-      g.dW = dW; g.dbh = dbh; g.partial = scratch;
+      g.dW = dW; g.dbh = dbh; g.dbi = dbi; g.partial = scratch;
       g.T = d.T; g.B = d.B; g.H = d.H; g.nb = d.nb; g.Hb = d.Hb;
       g.w_gate_stride = d.gate_stride; g.w_block_stride = d.block_stride; g.qin = qi;
       g.out_on_qin_grid = (qi.enabled && qo.enabled && qi.scale == qo.scale && qi.qmin == qo.qmin &&
@@ -388,7 +400,7 @@ static int scan_backward_impl(const b200gru_shape* shape, const float* gi, const
       }
       if (step_path(d)) {
         const tc::TcWeights w = {W, codes, scales};
-        return tc::launch_tc_dense_backward(h0, w, out, S, dout, dgi, dh0, dW, dbh, ws + s_off, d.T, d.B, d.H, qi, qo,
+        return tc::launch_tc_dense_backward(h0, w, out, S, dout, dgi, dh0, dW, dbh, dbi, ws + s_off, d.T, d.B, d.H, qi, qo,
                                             st);
       }
       const ScanPlan plan = plan_scan(d, false, codes != nullptr && scales != nullptr, qi);
@@ -416,7 +428,7 @@ static int scan_backward_impl(const b200gru_shape* shape, const float* gi, const
       if (tc_wgrad_path(d)) {
         // off-chain products on the tensor cores: bias sums first (their scratch leads), then dW
         char* sc = ws + s_off;
-        rc = launch_bias_grads(dgi, S, reinterpret_cast<float*>(sc), dbh, d.T, d.B, d.H, st);
+        rc = launch_bias_grads(dgi, S, reinterpret_cast<float*>(sc), dbh, dbi, d.T, d.B, d.H, st);
         if (rc) return rc;
         sc += align_up(bias_grads_scratch_bytes(d.T, d.B, d.H), 256);
         return tc::launch_tc_weight_grads(dgi, S, h0, out, qi, dW, sc, d.T, d.B, d.H, st);
@@ -453,7 +465,7 @@ static int scan_backward_impl(const b200gru_shape* shape, const float* gi, const
       a.dgi_c = dgi;
       rc = bfly_launch_wgrad(a, part_w, dW, st);
       if (rc) return rc;
-      return launch_bias_grads(dgi, S, part_b, dbh, d.T, d.B, d.H, st);
+      return launch_bias_grads(dgi, S, part_b, dbh, dbi, d.T, d.B, d.H, st);
     }
   }
   return B200GRU_INVALID_ARGUMENT;
@@ -464,8 +476,22 @@ int b200gru_scan_backward(const b200gru_shape* shape, const float* gi, const flo
                           const b200gru_quant* q_in, const b200gru_quant* q_out, float* dgi, float* dh0,
                           float* dW, float* dbh, void* workspace, size_t workspace_bytes_, void* stream) {
   return scan_backward_impl(shape, gi, h0, W, nullptr, nullptr, bh, out, dout, save, q_in, q_out, dgi, dh0, dW, dbh,
-                            workspace, workspace_bytes_, stream);
+                            nullptr, workspace, workspace_bytes_, stream);
 }
+
+}  // extern "C"
+
+namespace b200gru {
+int layer_scan_backward(const b200gru_shape* shape, const float* gi, const float* h0, const float* W, const signed char* codes,
+                        const float* scales, const float* bh, const float* out, const float* dout, const float* save,
+                        const b200gru_quant* q_in, const b200gru_quant* q_out, float* dgi, float* dh0, float* dW, float* dbh,
+                        float* dbi, void* workspace, size_t workspace_bytes_, void* stream) {
+  return scan_backward_impl(shape, gi, h0, W, codes, scales, bh, out, dout, save, q_in, q_out, dgi, dh0, dW, dbh, dbi, workspace,
+                            workspace_bytes_, stream);
+}
+}  // namespace b200gru
+
+extern "C" {
 
 // ---- per-kind conveniences ---------------------------------------------------
 
@@ -583,7 +609,7 @@ int b200gru_dense_q8_backward(const float* gi, const float* h0, const float* Wq,
   if (!codes || !scales) return B200GRU_INVALID_ARGUMENT;
   const b200gru_shape s = mk_shape(B200GRU_DENSE, T, B, H, 1, 0);
   return scan_backward_impl(&s, gi, h0, Wq, codes, scales, bh_cat, out, dout, save, q_in, q_out, dgi, dh0, dWq, dbh,
-                            workspace, workspace_bytes_, stream);
+                            nullptr, workspace, workspace_bytes_, stream);
 }
 
 void b200gru_test_select_dense_scan(int which) { g_test_choice[2].store(which, std::memory_order_relaxed); }

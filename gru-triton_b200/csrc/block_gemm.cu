@@ -14,6 +14,8 @@
 // FP32 FMA keeps the 1e-5 / 1e-4 parity budget; reductions are split over row
 // ranges into partial buffers and summed in a fixed order (bitwise reproducible).
 
+#include <cstring>
+
 #include "block_scan.cuh"
 #include "butterfly_scan.cuh"
 
@@ -309,33 +311,49 @@ weight_grads_kernel(const BlockGemmArgs a, float* __restrict__ dst, int rows_per
   }
 }
 
-// dbh: column sums of dgh over a range of rows; partial[split][3H]
+// Column sums over a range of rows: dgi of the three gates and dgh_n = dgi_n * r; partial[split][4][H].  One read of dgi
+// gives the gradients of both biases (their r and z parts are the same sums).  HBM bound: a thread keeps the 16
+// 16-byte loads of four rows in flight (one 4-byte load per thread before: 3 TB/s at T = B = 512, H = 1024).
+template <typename V>
+__device__ __forceinline__ V times(const V& a, const V& b);
+template <>
+__device__ __forceinline__ float times<float>(const float& a, const float& b) { return a * b; }
+template <>
+__device__ __forceinline__ float4 times<float4>(const float4& a, const float4& b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+__device__ __forceinline__ void plus(float& s, float v) { s += v; }
+__device__ __forceinline__ void plus(float4& s, const float4& v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+__device__ __forceinline__ void clear(float& s) { s = 0.f; }
+__device__ __forceinline__ void clear(float4& s) { s = make_float4(0.f, 0.f, 0.f, 0.f); }
+
+template <typename V>
 __global__ void __launch_bounds__(256)
-bias_grads_kernel(const float* __restrict__ dgi, const float* __restrict__ S, float* __restrict__ dst,
-                  int TB, int H, int rows_per_split) {
-  __shared__ float red[8][32];
+bias_grads_kernel(const V* __restrict__ dgi, const V* __restrict__ S, V* __restrict__ dst, int TB, int HV, int rows_per_split) {
+  __shared__ V red[8][4][32];
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col = blockIdx.x * 32 + lane;                  // in [0, 3H)
+  const int col = blockIdx.x * 32 + lane;                  // in [0, H / elements of V)
   const int r_begin = blockIdx.y * rows_per_split;
   const int r_end = min(TB, r_begin + rows_per_split);
-  float s = 0.f;
-  if (col < 3 * H) {
-    const bool is_n = col >= 2 * H;
+  V s[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) clear(s[k]);
+  if (col < HV) {
+#pragma unroll 4
     for (int tb = r_begin + warp; tb < r_end; tb += 8) {
-      float v = dgi[(size_t)tb * 3 * H + col];
-      if (is_n) v = v * S[(size_t)tb * H + (col - 2 * H)];
-      s += v;
+      const V* d = dgi + (size_t)tb * 3 * HV + col;
+      const V r = __ldcs(d), z = __ldcs(d + HV), n = __ldcs(d + 2 * HV), gate = __ldcs(S + (size_t)tb * HV + col);
+      plus(s[0], r); plus(s[1], z); plus(s[2], n); plus(s[3], times(n, gate));
     }
   }
-  red[warp][lane] = s;
-  __syncthreads();
-  if (warp == 0 && col < 3 * H) {
-    float t = red[0][lane];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) t += red[w][lane];
-    dst[(size_t)blockIdx.y * 3 * H + col] = t;
+  for (int k = 0; k < 4; ++k) red[warp][k][lane] = s[k];
+  __syncthreads();
+  if (warp < 4 && col < HV) {
+    V t = red[0][warp][lane];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) plus(t, red[w][warp][lane]);
+    dst[((size_t)blockIdx.y * 4 + warp) * HV + col] = t;
   }
 }
 
@@ -370,11 +388,11 @@ static WgPlan wg_plan(int T, int B, int nb, int Hb) {
   return p;
 }
 
-static void bg_splits(int T, int B, int* nsplit, int* rows_per_split) {
+// Row ranges of at least 32 rows, about four CTAs per SM in all.
+static void bg_splits(int T, int B, int H, int* nsplit, int* rows_per_split) {
   const int TB = T * B;
-  int s = cdiv(TB, 256);
-  if (s > 64) s = 64;
-  if (s < 1) s = 1;
+  int s = cdiv(4 * 148, cdiv(H, 128));
+  if (s > cdiv(TB, 32)) s = cdiv(TB, 32);
   const int rps = cdiv(TB, s);
   *nsplit = cdiv(TB, rps);
   *rows_per_split = rps;
@@ -382,41 +400,49 @@ static void bg_splits(int T, int B, int* nsplit, int* rows_per_split) {
 
 size_t bias_grads_scratch_bytes(int T, int B, int H) {
   int nsb, rpsb;
-  bg_splits(T, B, &nsb, &rpsb);
-  return align_up((size_t)nsb * 3 * H * sizeof(float), 256);
+  bg_splits(T, B, H, &nsb, &rpsb);
+  return align_up((size_t)nsb * 4 * H * sizeof(float), 256);
 }
 
-int launch_bias_grads(const float* dgi, const float* S, float* partial, float* dbh, int T, int B, int H,
+int launch_bias_grads(const float* dgi, const float* S, float* partial, float* dbh, float* dbi, int T, int B, int H,
                       cudaStream_t st) {
   int nsb, rpsb;
-  bg_splits(T, B, &nsb, &rpsb);
-  dim3 gridb(cdiv(3 * H, 32), nsb);
-  launch_pdl(bias_grads_kernel, gridb, dim3(256), 0, st, dgi, S, partial, T * B, H, rpsb);
+  bg_splits(T, B, H, &nsb, &rpsb);
+  const uintptr_t any = reinterpret_cast<uintptr_t>(dgi) | reinterpret_cast<uintptr_t>(S) | reinterpret_cast<uintptr_t>(partial);
+  if (H % 4 == 0 && (any & 15u) == 0)
+    launch_pdl(bias_grads_kernel<float4>, dim3(cdiv(H, 128), nsb), dim3(256), 0, st, reinterpret_cast<const float4*>(dgi),
+               reinterpret_cast<const float4*>(S), reinterpret_cast<float4*>(partial), T * B, H / 4, rpsb);
+  else
+    launch_pdl(bias_grads_kernel<float>, dim3(cdiv(H, 32), nsb), dim3(256), 0, st, dgi, S, partial, T * B, H, rpsb);
   note_launch();
   int rc = check_launch("bias_grads_kernel");
   if (rc) return rc;
-  launch_reduce_partials(partial, nsb, (size_t)3 * H, (size_t)3 * H, dbh, st);
+  ReduceTargets t;
+  memset(&t, 0, sizeof(t));
+  const size_t h = H;
+  t.add(0, 2 * h, dbh, dbi);
+  if (dbi != nullptr) t.add(2 * h, 3 * h, dbi + 2 * h, nullptr);
+  t.add(3 * h, 4 * h, dbh + 2 * h, nullptr);
+  launch_reduce_targets(partial, nsb, 4 * h, 4 * h, t, st);
   return check_launch("reduce_partials");
 }
 
 size_t weight_grads_scratch_bytes(int T, int B, int H, int nb, int Hb) {
   int nsb, rpsb;
   const int ns = wg_plan(T, B, nb, Hb).nsplit;
-  bg_splits(T, B, &nsb, &rpsb);
+  bg_splits(T, B, H, &nsb, &rpsb);
   size_t f = 0;
   if (ns > 1) f += (size_t)ns * 3 * nb * Hb * Hb;
-  f += (size_t)nsb * 3 * H;
+  f += (size_t)nsb * 4 * H + 4;                            // the bias sums start on a 16-byte boundary
   return align_up(f * sizeof(float), 256);
 }
 
 int launch_weight_grads(const BlockGemmArgs& a, cudaStream_t st) {
-  int nsb, rpsb;
   const WgPlan p = wg_plan(a.T, a.B, a.nb, a.Hb);
   const int ns = p.nsplit;
-  bg_splits(a.T, a.B, &nsb, &rpsb);
   const size_t dw_elems = (size_t)3 * a.nb * a.Hb * a.Hb;
   float* part_w = a.partial;
-  float* part_b = a.partial + (ns > 1 ? (size_t)ns * dw_elems : 0);
+  float* part_b = a.partial + (ns > 1 ? ((size_t)ns * dw_elems + 3) / 4 * 4 : 0);
   float* dst = ns > 1 ? part_w : a.dW;
 
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
@@ -437,7 +463,7 @@ int launch_weight_grads(const BlockGemmArgs& a, cudaStream_t st) {
   if (rc) return rc;
   if (ns > 1) launch_reduce_partials(part_w, ns, dw_elems, dw_elems, a.dW, st);
 
-  return launch_bias_grads(a.dgi, a.S, part_b, a.dbh, a.T, a.B, a.H, st);
+  return launch_bias_grads(a.dgi, a.S, part_b, a.dbh, a.dbi, a.T, a.B, a.H, st);
 }
 
 }  // namespace b200gru

@@ -64,6 +64,7 @@ struct BlockGemmArgs {
   float* S;            // recompute_gates: written; weight_grads: read
   float* dW;
   float* dbh;
+  float* dbi;          // optional: column sums of dgi as well
   float* partial;      // scratch for split reductions
   int T, B, H, nb, Hb;
   long long w_gate_stride, w_block_stride;

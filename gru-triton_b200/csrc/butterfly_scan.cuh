@@ -55,7 +55,7 @@ int bfly_launch_wgrad(BflyArgs a, float* partial, float* dtw, cudaStream_t st);
 
 // block_gemm.cu: bias gradient (shared by dense, block-diagonal and butterfly)
 size_t bias_grads_scratch_bytes(int T, int B, int H);
-int launch_bias_grads(const float* dgi, const float* S, float* partial, float* dbh, int T, int B, int H,
+int launch_bias_grads(const float* dgi, const float* S, float* partial, float* dbh, float* dbi, int T, int B, int H,
                       cudaStream_t st);
 
 }  // namespace b200gru

@@ -196,6 +196,25 @@ int allow_dynamic_smem(const void* kernel, size_t bytes);
 // dst[i] = src[0*row_stride + i] + src[1*row_stride + i] + ... (fixed order).
 void launch_reduce_partials(const float* src, int nparts, size_t row_stride, size_t n, float* dst,
                             cudaStream_t st);
+// The same with several destinations: columns [begin, end) of the sum go to a and, where given, to b as well.
+struct ReduceTargets {
+  static constexpr int MAX = 4;
+  int count;
+  size_t begin[MAX], end[MAX];
+  float* a[MAX];
+  float* b[MAX];
+  void add(size_t from, size_t to, float* dst, float* copy) {
+    begin[count] = from; end[count] = to; a[count] = dst; b[count] = copy; ++count;
+  }
+};
+void launch_reduce_targets(const float* src, int nparts, size_t row_stride, size_t n, const ReduceTargets& t, cudaStream_t st);
+
+// b200gru_scan_backward with optional int8 weight codes and, where dbi is given, the column sums of dgi as well
+// (the gradient of the input bias): its r and z parts are those of dbh.
+int layer_scan_backward(const b200gru_shape* shape, const float* gi, const float* h0, const float* W, const signed char* codes,
+                        const float* scales, const float* bh, const float* out, const float* dout, const float* save,
+                        const b200gru_quant* q_in, const b200gru_quant* q_out, float* dgi, float* dh0, float* dW, float* dbh,
+                        float* dbi, void* workspace, size_t workspace_bytes, void* stream);
 
 // ---- programmatic dependent launch ---------------------------------------------------------------
 // The per-step kernels of a scan form a chain in one stream; each is launched with the

@@ -15,6 +15,8 @@
 #include <cstdlib>
 #include <mutex>
 
+#include <cstring>
+
 #include "common.cuh"
 
 namespace b200gru {
@@ -272,16 +274,16 @@ diag_bwd_kernel(const float* __restrict__ gi, const float* __restrict__ h0,
                 const float* __restrict__ W, const float* __restrict__ bh,
                 const float* __restrict__ out, const float* __restrict__ dout,
                 float* __restrict__ dgi, float* __restrict__ dh0,
-                float* __restrict__ partial, int T, int B, int H, Quant qin, Quant qout) {
+                float* __restrict__ partial, int nsums, int T, int B, int H, Quant qin, Quant qout) {
   const int hv = H / VEC;
   const int iv = blockIdx.x * 32 + threadIdx.x;
   const int b = blockIdx.y * DIAG_BY + threadIdx.y;
   const bool active = (iv < hv) && (b < B);
   const int i = iv * VEC;
 
-  float acc[6][VEC];
+  float acc[7][VEC];
 #pragma unroll
-  for (int k = 0; k < 6; ++k)
+  for (int k = 0; k < 7; ++k)
 #pragma unroll
     for (int v = 0; v < VEC; ++v) acc[k][v] = 0.f;
 
@@ -343,6 +345,7 @@ diag_bwd_kernel(const float* __restrict__ gi, const float* __restrict__ h0,
             acc[3][v] += q.dgr;
             acc[4][v] += q.dgz;
             acc[5][v] += q.dghn;
+            acc[6][v] += q.dgn;
             float via = q.dgr * wr[v] + q.dgz * wz[v] + q.dghn * wn[v];
             via = via * ste_mask<QIN>(h_prev, qin);
             dh_acc[v] = via + q.dh_direct;
@@ -365,16 +368,17 @@ diag_bwd_kernel(const float* __restrict__ gi, const float* __restrict__ h0,
     st_vec<VEC>(dh0 + (size_t)b * H + i, dh_acc);
   }
 
-  // reduce the six sums over the BY rows of this block (fixed order), one partial row out
-  __shared__ float red[DIAG_BY][6][32 * VEC];
+  // reduce the sums over the BY rows of this block (fixed order), one partial row out
+  __shared__ float red[DIAG_BY][7][32 * VEC];
 #pragma unroll
-  for (int k = 0; k < 6; ++k)
+  for (int k = 0; k < 7; ++k)
 #pragma unroll
     for (int v = 0; v < VEC; ++v) red[threadIdx.y][k][threadIdx.x * VEC + v] = acc[k][v];
   __syncthreads();
   if (threadIdx.y == 0 && iv < hv) {
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
+    for (int k = 0; k < 7; ++k) {
+      if (k >= nsums) break;
       float s[VEC];
 #pragma unroll
       for (int v = 0; v < VEC; ++v) {
@@ -383,7 +387,7 @@ diag_bwd_kernel(const float* __restrict__ gi, const float* __restrict__ h0,
         for (int y = 1; y < DIAG_BY; ++y) a += red[y][k][threadIdx.x * VEC + v];
         s[v] = a;
       }
-      st_vec<VEC>(partial + ((size_t)blockIdx.y * 6 + k) * H + i, s);
+      st_vec<VEC>(partial + ((size_t)blockIdx.y * nsums + k) * H + i, s);
     }
   }
 }
@@ -403,9 +407,9 @@ static int pick_vec(int B, int H, bool ptr_ok) {
   return 1;
 }
 
-size_t diag_bwd_workspace_bytes(int T, int B, int H) {
+size_t diag_bwd_workspace_bytes(int T, int B, int H, bool input_bias) {
   (void)T;
-  return align_up((size_t)cdiv(B, DIAG_BY) * 6 * H * sizeof(float), 256);
+  return align_up((size_t)cdiv(B, DIAG_BY) * (input_bias ? 7 : 6) * H * sizeof(float), 256);
 }
 
 template <int VEC, int PF>
@@ -449,13 +453,13 @@ int diag_forward(const float* gi, const float* h0, const float* W, const float* 
 
 template <int VEC, int PF>
 static void launch_bwd(const float* gi, const float* h0, const float* W, const float* bh,
-                       const float* out, const float* dout, float* dgi, float* dh0, float* partial,
+                       const float* out, const float* dout, float* dgi, float* dh0, float* partial, int nsums,
                        int T, int B, int H, Quant qi, Quant qo, cudaStream_t st) {
   dim3 block(32, DIAG_BY);
   dim3 grid(cdiv(H / VEC, 32), cdiv(B, DIAG_BY));
 #define DIAG_BWD(QI, QO)                                                                     \
   diag_bwd_kernel<VEC, PF, QI, QO><<<grid, block, 0, st>>>(gi, h0, W, bh, out, dout, dgi, dh0, \
-                                                           partial, T, B, H, qi, qo)
+                                                           partial, nsums, T, B, H, qi, qo)
   if (qi.enabled) { if (qo.enabled) DIAG_BWD(true, true); else DIAG_BWD(true, false); }
   else            { if (qo.enabled) DIAG_BWD(false, true); else DIAG_BWD(false, false); }
 #undef DIAG_BWD
@@ -463,22 +467,28 @@ static void launch_bwd(const float* gi, const float* h0, const float* W, const f
 }
 
 int diag_backward(const float* gi, const float* h0, const float* W, const float* bh,
-                  const float* out, const float* dout, float* dgi, float* dh0, float* dW, float* dbh,
+                  const float* out, const float* dout, float* dgi, float* dh0, float* dW, float* dbh, float* dbi,
                   void* workspace, int T, int B, int H, Quant qi, Quant qo, cudaStream_t st) {
   float* partial = static_cast<float*>(workspace);
+  const int nsums = dbi != nullptr ? 7 : 6;                        // the seventh: sums of dgi_n
   if (cdiv(B, DIAG_BY) > 65535) return B200GRU_UNSUPPORTED;        // grid.y of the backward kernel
   const bool ok = aligned16(gi) && aligned16(h0) && aligned16(W) && aligned16(bh) && aligned16(out) &&
                   aligned16(dout) && aligned16(dgi) && aligned16(dh0) && aligned16(partial);
   const int vec = pick_vec(B, H, ok);
-  if (vec == 4) launch_bwd<4, 2>(gi, h0, W, bh, out, dout, dgi, dh0, partial, T, B, H, qi, qo, st);
-  else if (vec == 2) launch_bwd<2, 3>(gi, h0, W, bh, out, dout, dgi, dh0, partial, T, B, H, qi, qo, st);
-  else launch_bwd<1, 4>(gi, h0, W, bh, out, dout, dgi, dh0, partial, T, B, H, qi, qo, st);
+  if (vec == 4) launch_bwd<4, 2>(gi, h0, W, bh, out, dout, dgi, dh0, partial, nsums, T, B, H, qi, qo, st);
+  else if (vec == 2) launch_bwd<2, 3>(gi, h0, W, bh, out, dout, dgi, dh0, partial, nsums, T, B, H, qi, qo, st);
+  else launch_bwd<1, 4>(gi, h0, W, bh, out, dout, dgi, dh0, partial, nsums, T, B, H, qi, qo, st);
   int rc = check_launch("diag_bwd_kernel");
   if (rc) return rc;
-  // partial[part][0..2][H] -> dW[3][H];  partial[part][3..5][H] -> dbh[3H]
-  const int nparts = cdiv(B, DIAG_BY);
-  launch_reduce_partials(partial, nparts, (size_t)6 * H, (size_t)3 * H, dW, st);
-  launch_reduce_partials(partial + (size_t)3 * H, nparts, (size_t)6 * H, (size_t)3 * H, dbh, st);
+  // partial[part][0..2][H] -> dW[3][H];  partial[part][3..5][H] -> dbh[3H];  dbi: the sums of r and z, and the seventh
+  const size_t h = H;
+  ReduceTargets t;
+  memset(&t, 0, sizeof(t));
+  t.add(0, 3 * h, dW, nullptr);
+  t.add(3 * h, 5 * h, dbh, dbi);
+  t.add(5 * h, 6 * h, dbh + 2 * h, nullptr);
+  if (dbi != nullptr) t.add(6 * h, 7 * h, dbi + 2 * h, nullptr);
+  launch_reduce_targets(partial, cdiv(B, DIAG_BY), nsums * h, nsums * h, t, st);
   return check_launch("reduce_partials");
 }
 
@@ -528,13 +538,13 @@ extern "C" int b200gru_diagonal_backward_noalloc(const float* gi, const float* h
   if (T <= 0 || B <= 0 || H <= 0) return B200GRU_INVALID_ARGUMENT;
   if (q_in && q_in->enabled && !(q_in->scale > 0.f)) return B200GRU_INVALID_ARGUMENT;
   if (q_out && q_out->enabled && !(q_out->scale > 0.f)) return B200GRU_INVALID_ARGUMENT;
-  if (diag_bwd_workspace_bytes(T, B, H) > (size_t)B200GRU_NOALLOC_SCRATCH_BYTES) return B200GRU_SCRATCH_EXCEEDED;
+  if (diag_bwd_workspace_bytes(T, B, H, false) > (size_t)B200GRU_NOALLOC_SCRATCH_BYTES) return B200GRU_SCRATCH_EXCEEDED;
   if (cdiv(B, DIAG_BY) > 65535) return B200GRU_UNSUPPORTED;        // grid.y of the backward kernel
   float* scratch = nullptr;
   const int rc = noalloc_scratch_address(&scratch);
   if (rc) return rc;
   // Every element of the scratch that the reduction reads is first written by this call's
   // backward kernel, so nothing has to be cleared; what an earlier call left is ignored.
-  return diag_backward(gi, h0, Wh_diag, bh_cat, out, dout, dgi, dh0, dWh_diag, dbh, scratch, T, B, H,
+  return diag_backward(gi, h0, Wh_diag, bh_cat, out, dout, dgi, dh0, dWh_diag, dbh, nullptr, scratch, T, B, H,
                        make_quant(q_in), make_quant(q_out), static_cast<cudaStream_t>(stream));
 }

@@ -291,20 +291,19 @@ LinearPlan linear_plan(const Layer& L) {
   p.dyp = pad(2 * chunk * n3 * 2);
   p.xp = pad(2 * chunk * L.I * 2);
   p.acc = pad((size_t)p.splits * n3 * L.I * 4);
-  p.sums = pad(column_sums_scratch_bytes(L.rows, 3 * L.H)) + pad(column_sums_scratch_bytes(p.splits, (int)(n3 * L.I)));
+  p.sums = pad(column_sums_scratch_bytes(p.splits, (int)(n3 * L.I)));
   p.total = p.dyp + p.xp + p.acc + p.sums;
   return p;
 }
 
-// dWi, db_i, dx from dgi (dWi / dx / db_i may be NULL: not wanted)
-int linear_backward(const Layer& L, const Kept& k, const float* x, const float* dgi, float* dWi, float* dbi, float* dx,
+// dWi, dx from dgi (either may be NULL: not wanted)
+int linear_backward(const Layer& L, const Kept& k, const float* x, const float* dgi, float* dWi, float* dx,
                     char* ws, cudaStream_t st) {
   const LinearPlan p = linear_plan(L);
   char* dyp = ws; ws += p.dyp;
   char* xp = ws; ws += p.xp;
   float* acc = reinterpret_cast<float*>(ws); ws += p.acc;
   float* sums = reinterpret_cast<float*>(ws);
-  float* sums2 = reinterpret_cast<float*>(ws + pad(column_sums_scratch_bytes(L.rows, 3 * L.H)));
   const int n3 = 3 * L.H;
   const size_t w = (size_t)n3 * L.I;
   int rc = B200GRU_OK;
@@ -350,11 +349,10 @@ int linear_backward(const Layer& L, const Kept& k, const float* x, const float* 
   }
   if (dWi != nullptr) {
     float* full = L.bits_i <= 8 ? acc : dWi;                 // slice 0 is overwritten by the sum when it has to be
-    if (p.splits > 1) rc = launch_column_sums(acc, p.splits, (int)w, full, sums2, st);
+    if (p.splits > 1) rc = launch_column_sums(acc, p.splits, (int)w, full, sums, st);
     if (!rc && L.bits_i <= 8) rc = launch_quantize_rows_backward(k.Wi, full, n3, L.I, L.bits_i, dWi, st);
     if (rc) return rc;
   }
-  if (dbi != nullptr) rc = launch_column_sums(dgi, L.rows, n3, dbi, sums, st);
   return rc;
 }
 
@@ -438,17 +436,13 @@ int b200gru_layer_backward(const int* dims, const float* quants, const void* con
   float* dWq = nullptr;
   if (L.bits_h <= 8) { dWq = reinterpret_cast<float*>(scratch); scratch += pad(L.w_elems * 4); }
   int rc;                               // gi is read only where the gates were not saved; dgi stands in for it
-  if (L.bits_h <= 8) {
-    rc = b200gru_dense_q8_backward(dgi, h0, k.Wh_q, k.Wh_codes, k.Wh_scale, k.b_h, out, dout, save, L.T, L.B, L.H, &qi, &qo,
-                                   dgi, o[1], dWq, o[5], scratch, scan_ws(L, 2), stream);
-    if (!rc) rc = launch_quantize_rows_backward(k.Wh, dWq, 3 * L.H, L.H, L.bits_h, o[3], st);
-  } else {
-    const bool gi_in = keeps_gi(L);
-    rc = b200gru_scan_backward(&L.shape, gi_in ? save : dgi, h0, k.Wh, k.b_h, out, dout, gi_in ? nullptr : save, &qi, &qo,
-                               dgi, o[1], o[3], o[5], scratch, scan_ws(L, gi_in ? 1 : 2), stream);
-  }
+  const bool q8 = L.bits_h <= 8, gi_in = keeps_gi(L);
+  rc = layer_scan_backward(&L.shape, gi_in ? save : dgi, h0, q8 ? k.Wh_q : k.Wh, k.Wh_codes, q8 ? k.Wh_scale : nullptr, k.b_h, out, dout,
+                           gi_in ? nullptr : save, &qi, &qo, dgi, o[1], q8 ? dWq : o[3], o[5], o[4], scratch,
+                           scan_ws(L, gi_in ? 1 : 2), stream);
+  if (!rc && q8) rc = launch_quantize_rows_backward(k.Wh, dWq, 3 * L.H, L.H, L.bits_h, o[3], st);
   if (rc) return rc;
-  return linear_backward(L, k, x, dgi, o[2], o[4], o[0], scratch, st);
+  return linear_backward(L, k, x, dgi, o[2], o[0], scratch, st);
 }
 
 }  // extern "C"

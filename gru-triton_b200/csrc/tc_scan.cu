@@ -458,7 +458,7 @@ int launch_tc_dense_forward(const float* gi, const float* h0, const TcWeights& w
 }
 
 int launch_tc_dense_backward(const float* h0, const TcWeights& w, const float* out, const float* S, const float* dout,
-                             float* dgi, float* dh0, float* dW, float* dbh, void* scratch, int T, int B, int H,
+                             float* dgi, float* dh0, float* dW, float* dbh, float* dbi, void* scratch, int T, int B, int H,
                              Quant qin, Quant qout, cudaStream_t st) {
   const Plan p = make_plan(T, B, H, w.codes != nullptr, qin);
   const size_t rows = (size_t)p.tc_steps * B;
@@ -557,7 +557,7 @@ int launch_tc_dense_backward(const float* h0, const TcWeights& w, const float* o
   rc = check_launch("dh0_kernel");
   if (rc) return rc;
   if (p.dw_splits > 1) launch_reduce_partials(dw_part, p.dw_splits, (size_t)3 * H * H, (size_t)3 * H * H, dW, st);
-  return launch_bias_grads(dgi, S, bias_part, dbh, T, B, H, st);
+  return launch_bias_grads(dgi, S, bias_part, dbh, dbi, T, B, H, st);
 }
 
 

@@ -23,7 +23,7 @@ int launch_tc_dense_forward(const float* gi, const float* h0, const TcWeights& w
                             float* save, void* scratch, int T, int B, int H, Quant qin, Quant qout, cudaStream_t st);
 // dW is the gradient with respect to the weight VALUES (for codes: codes * row_scale).
 int launch_tc_dense_backward(const float* h0, const TcWeights& w, const float* out, const float* S, const float* dout,
-                             float* dgi, float* dh0, float* dW, float* dbh, void* scratch, int T, int B, int H,
+                             float* dgi, float* dh0, float* dW, float* dbh, float* dbi, void* scratch, int T, int B, int H,
                              Quant qin, Quant qout, cudaStream_t st);
 
 // Weight gradient of the dense scan as one tensor-core product over all T*B rows (used after the
