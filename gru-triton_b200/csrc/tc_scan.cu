@@ -531,7 +531,11 @@ int launch_tc_dense_backward(const float* h0, const TcWeights& w, const float* o
     a.via = (t == T - 1) ? nullptr : via;
     a.h_t = out + (size_t)t * B * H;
     a.h_prev = (t == 0) ? h0 : out + (size_t)(t - 1) * B * H;
-    launch_pdl(gate_bwd_kernel, dim3(cdiv(n4, 256)), dim3(256), 0, st, a);
+    // The gate kernel reads dout, S and out before it waits for its predecessor.  That is safe behind the chain product,
+    // but the first one follows a weight preparation that may itself have started while the forward's last
+    // step or the producer of dout still runs: it is launched with a full dependency.
+    if (t == T - 1) gate_bwd_kernel<<<cdiv(n4, 256), 256, 0, st>>>(a);
+    else launch_pdl(gate_bwd_kernel, dim3(cdiv(n4, 256)), dim3(256), 0, st, a);
     note_launch();
     gv.A = dgh_op + (size_t)slot * B * 3 * H;
     rc = launch_tc_gemm(gv, st);

@@ -330,6 +330,31 @@ def test_zz_bounded_wait_gives_up_and_is_reported():
     _lib.check_device_status()
 
 
+def test_step_path_backward_right_behind_its_forward():
+    """The first backward kernel reads what the forward's last step writes: back to back calls on changing inputs give
+    the bits of calls that are waited for."""
+    from gru_triton_b200 import _lib
+    T, B, H = 3, 257, 608
+    g = torch.Generator(device="cuda").manual_seed(2)
+    W = torch.empty(3 * H, H, device="cuda").uniform_(-0.04, 0.04, generator=g)
+    bh = torch.zeros(3 * H, device="cuda")
+    sets = [[torch.randn(s, device="cuda", generator=g) for s in ((T, B, 3 * H), (B, H), (T, B, H))] for _ in range(6)]
+    def call(gi, h0, dout, wait):
+        out, save = _lib.scan_forward("dense", gi, h0, W, bh, None, None, want_save=True)
+        if wait:
+            torch.cuda.synchronize()
+        grads = _lib.scan_backward("dense", gi, h0, W, bh, out, dout, save, None, None)
+        if wait:
+            torch.cuda.synchronize()
+        return (out, *grads)
+    waited = [call(*s, True) for s in sets]
+    for _ in range(3):
+        behind = [call(*s, False) for s in sets]
+        torch.cuda.synchronize()
+        for a, b in zip(waited, behind):
+            assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
 @pytest.mark.parametrize("dtype,M,N,K,pa,pb,a_mn,b_mn,split", [
     ("f16", 256, 256, 64, 1, 1, False, False, 1), ("f16", 300, 520, 200, 2, 2, False, False, 1),
     ("bf16", 136, 264, 1024, 2, 2, True, True, 1), ("bf16", 513, 304, 520, 3, 3, False, True, 1),
