@@ -162,7 +162,8 @@ codes_to_f16_kernel(const signed char* __restrict__ src, __half* __restrict__ ds
   d[1] = __halves2half2(__float2half_rn((float)c.z), __float2half_rn((float)c.w));
 }
 
-// x -> integer codes of a frozen quantiser, exact in fp16
+// x -> integer codes of a frozen quantiser, exact in fp16.  A NaN stays one: the clamp would make a code of it, and a
+// broken frame would come out as ordinary numbers.
 __global__ void __launch_bounds__(256)
 quantize_to_f16_kernel(const float* __restrict__ x, __half* __restrict__ dst, size_t n4, Quant q) {
   pdl_launch_dependents();
@@ -173,7 +174,7 @@ quantize_to_f16_kernel(const float* __restrict__ x, __half* __restrict__ dst, si
   const float e[4] = {v.x, v.y, v.z, v.w};
   __half h[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) h[k] = __float2half_rn(fminf(fmaxf(fq_code(e[k], q), q.qmin), q.qmax));
+  for (int k = 0; k < 4; ++k) h[k] = __float2half_rn(e[k] == e[k] ? fminf(fmaxf(fq_code(e[k], q), q.qmin), q.qmax) : e[k]);
   __half2* d = reinterpret_cast<__half2*>(dst) + 2 * i;
   d[0] = __halves2half2(h[0], h[1]);
   d[1] = __halves2half2(h[2], h[3]);

@@ -479,3 +479,37 @@ def test_layer_entry_leaves_other_forms_to_the_composed_path():
         assert layer_native.forward(layer, x, h0) is None
     odd = gru.GRULayer(41, 64, fp32, gate_layout="fused").cuda()
     assert layer_native.forward(odd, torch.randn(2, 3, 41, device="cuda"), h0) is None
+
+
+def _layer(I, H, *, kind=None, wbits=32, xbits=32, hbits=32, seed=3, **kw):
+    """A fused layer on the GPU with its activation quantisers frozen."""
+    import gru_triton_b200 as gru
+    recipe = gru.QuantRecipe(weight=gru.QuantizerConfig(bits=wbits, axis=0), input_act=gru.QuantizerConfig(bits=xbits),
+                             hidden=gru.QuantizerConfig(bits=hbits))
+    struct = None if kind is None else gru.StructureConfig(kind=kind, nblocks=4, butterfly_nblocks=1)
+    torch.manual_seed(seed)
+    layer = gru.GRULayer(I, H, recipe, gate_layout="fused", structure_hidden=struct, **kw).cuda()
+    for q, s in ((layer.cell.quant_x, 0.03), (layer.cell.quant_h_in, 1 / 127.0), (layer.cell.quant_h_out, 1 / 127.0)):
+        q.scale = torch.tensor(s, device="cuda")
+        q.freeze()
+    return layer
+
+
+@pytest.mark.parametrize("wbits,hbits", [(32, 32), (8, 32), (32, 8), (8, 8)])
+def test_layer_entry_keeps_a_nan_of_a_quantised_input(wbits, hbits, monkeypatch):
+    """A NaN in x is no code of the input quantiser: it reaches every unit of its sequence from its frame on (an
+    int8 state maps it to a code, as the composed path does).  Infinities are the grid's ends."""
+    from gru_triton_b200 import layer_native
+    layer = _layer(40, 64, wbits=wbits, xbits=8, hbits=hbits)
+    x = torch.randn(4, 6, 40, device="cuda")
+    x[1, 1, 7], x[1, 3, 0], x[2, 4, 39] = float("nan"), float("inf"), float("-inf")
+    h0 = torch.zeros(6, 64, device="cuda")
+    with torch.no_grad():
+        native = layer_native.forward(layer, x, h0)
+        monkeypatch.setattr(layer_native, "forward", lambda *a: None)
+        composed, _ = layer(x, h0)
+    assert native is not None and torch.equal(native.isnan(), composed.isnan())
+    if hbits == 32:
+        assert bool(native[1:, 1].isnan().all()) and not bool(native[:, [0, 2, 3, 4, 5]].isnan().any())
+    ok = ~composed.isnan()
+    assert float((native[ok] - composed[ok]).norm()) <= (1e-2 if hbits == 8 else 2e-5) * float(composed[ok].norm())
