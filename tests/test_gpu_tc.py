@@ -513,3 +513,53 @@ def test_layer_entry_keeps_a_nan_of_a_quantised_input(wbits, hbits, monkeypatch)
         assert bool(native[1:, 1].isnan().all()) and not bool(native[:, [0, 2, 3, 4, 5]].isnan().any())
     ok = ~composed.isnan()
     assert float((native[ok] - composed[ok]).norm()) <= (1e-2 if hbits == 8 else 2e-5) * float(composed[ok].norm())
+
+
+# Two fp16 planes carry 22 bits of an operand (2 * 2^-23 of a term), and at most 32 steps of a truncating accumulator
+# lose 32 * 2^-24 of the largest partial sum: 2.2e-6 in all, of the largest entry of a product.
+PRODUCT_TOL = 4e-6
+
+
+@pytest.mark.parametrize("size", [0.04, 1e-4, 1e-6])
+@pytest.mark.parametrize("B,H", [(8, 64), (5, 512), (128, 608)])
+def test_hidden_gradient_with_a_zero_weight_row(B, H, size):
+    """A pruned row of the hidden weights contributes nothing to dgh . W and takes no precision from the others.  The
+    update gate is shut (z = 1e-13), so that dh0 is that product alone."""
+    from gru_triton_b200 import _lib
+    g = torch.Generator().manual_seed(H)
+    gi, h0, dout = (torch.randn(s, generator=g) for s in ((1, B, 3 * H), (B, H), (1, B, H)))
+    gi[..., H:2 * H] = -30.0
+    W = (torch.rand(3 * H, H, generator=g) * 2 - 1) * size
+    W[2 * H + 1] = 0.0
+    bh = torch.zeros(3 * H)
+    h = h0.double().requires_grad_(True)
+    gr, gz, gn = gi[0].double().chunk(3, -1)
+    hr, hz, hn = (h @ W.double().t()).chunk(3, -1)
+    z, n = torch.sigmoid(gz + hz), torch.tanh(gn + torch.sigmoid(gr + hr) * hn)
+    ((1 - z) * n + z * h).backward(dout[0].double())
+    d = [t.cuda() for t in (gi, h0, W, bh, dout)]
+    _lib.load().b200gru_test_select_dense_scan(2 if B < 128 else 0)
+    try:
+        out, save = _lib.scan_forward("dense", *d[:4], None, None, want_save=True)
+        dh0 = _lib.scan_backward("dense", *d[:4], out, d[4], save, None, None)[1]
+        torch.cuda.synchronize()
+    finally:
+        _lib.load().b200gru_test_select_dense_scan(0)
+    assert rel_err(dh0.cpu(), h.grad) <= PRODUCT_TOL
+
+
+@pytest.mark.parametrize("size", [0.04, 1e-4, 1e-6])
+def test_input_gradient_with_a_zero_weight_row(size):
+    """The same for dgi . Wi of a layer call, against the layer in 64 bits."""
+    layer = _layer(40, 64)
+    with torch.no_grad():
+        for gate in "rzn":
+            w = getattr(layer.cell, f"W_i{gate}")
+            w.copy_((torch.rand_like(w) * 2 - 1) * size)
+        layer.cell.W_in[3] = 0.0
+    ref = copy.deepcopy(layer).cpu().double()
+    x, h0, dout = torch.randn(2, 5, 40), torch.randn(5, 64) * 0.1, torch.randn(2, 5, 64)
+    xr, xg = x.double().requires_grad_(True), x.cuda().requires_grad_(True)
+    ref(xr, h0.double())[0].backward(dout.double())
+    layer(xg, h0.cuda())[0].backward(dout.cuda())
+    assert rel_err(xg.grad.cpu(), xr.grad) <= PRODUCT_TOL
