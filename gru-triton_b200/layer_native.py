@@ -3,7 +3,7 @@
 ``forward(layer, x, h0)`` runs the input projection and the scan of a dispatchable ``GRULayer`` with
 a dense input side and returns ``out``, or ``None`` where the call has a form this path does not take
 (other dtypes or devices, widths that are no multiple of 8, quantizers other than the kinds the
-kernels implement, tracing and function transforms): the caller then goes through the composed path
+kernels implement or with hooks, tracing and function transforms): the caller then goes through the composed path
 of ``tc.linear`` and the scan functions, which also words the errors.
 
 One step of one sequence (T = B = 1, 256 x 256) spent 190 us in the composed path's Python: four
@@ -18,7 +18,7 @@ from functools import lru_cache
 import torch
 
 from . import _lib
-from .quantizers import FakeQuantizePerChannel, Identity
+from .quantizers import FakeQuantizePerChannel, FakeQuantizePerGroup, FakeQuantizePerTensor, Identity
 
 _INTS = ctypes.c_int * 10
 _FLOATS = ctypes.c_float * 12
@@ -26,6 +26,7 @@ _FWD_PTRS = ctypes.c_void_p * 19
 _BWD_PTRS = ctypes.c_void_p * 14
 _SIZES = ctypes.c_size_t * 3
 _GATES = "rzn"
+_INPUT_QUANTIZERS = (Identity, FakeQuantizePerTensor, FakeQuantizePerChannel, FakeQuantizePerGroup)
 
 
 @lru_cache(maxsize=512)
@@ -58,6 +59,12 @@ def _weight_bits(quantizers):
                 cfg.bits != bits or bits > 8):
             return None
     return int(bits)
+
+
+def _observed(module) -> bool:
+    """The module has hooks, or a ``forward`` of the instance's own: it has to be called, once."""
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks or
+                "forward" in module.__dict__)
 
 
 def _plain(t, shape, device):
@@ -196,29 +203,35 @@ def forward(layer, x, h0):
             x.shape[2] != I or h0.dim() != 2 or h0.shape[0] != x.shape[1] or h0.shape[1] != H or _transformed()):
         return None
     mods = cell._modules
-    bits_i = _weight_bits([mods["quant_W_i" + g] for g in _GATES])
-    bits_h = _weight_bits([mods["quant_W_h" + g] for g in _GATES]) if kind == "dense" else 32
+    quant_x, quant_wi, quant_wh = mods["quant_x"], [mods["quant_W_i" + g] for g in _GATES], [mods["quant_W_h" + g] for g in _GATES]
+    bits_i = _weight_bits(quant_wi)
+    bits_h = _weight_bits(quant_wh) if kind == "dense" else 32
     if bits_i is None or bits_h is None:
+        return None
+    # the composed path calls the input quantizer and, where they are identities, those of dense hidden weights: these are
+    # passed by only where nobody could tell
+    if (type(quant_x) not in _INPUT_QUANTIZERS or torch.nn.modules.module._has_any_global_hook() or _observed(quant_x) or
+            (kind == "dense" and bits_h == 32 and any(map(_observed, quant_wh)))):
         return None
     found = _parameters(cell, kind, device, I, H)
     if found is None:
         return None
     params, nblocks, log2_hpad = found
+    T, B = x.shape[0], x.shape[1]
+    key = (kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h)
+    if _plan(*key) is None:
+        return None
     grad = torch.is_grad_enabled() and (x.requires_grad or h0.requires_grad or any([p.requires_grad for p in params]))
     qx = None
-    quant_x = mods["quant_x"]
     if type(quant_x) is not Identity:
-        qx = None if grad else _extract_h_quant_params(quant_x)
+        if type(quant_x) is FakeQuantizePerTensor and not grad:
+            qx = _extract_h_quant_params(quant_x)
         if qx is None or qx[1] < -127 or qx[2] > 127:
             qx, x = None, quant_x(x)
             if not _plain_input(x, device):
                 return None
     x, h0 = x.contiguous(), h0.contiguous()
     if x.data_ptr() & 15:
-        return None
-    T, B = x.shape[0], x.shape[1]
-    key = (kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h)
-    if _plan(*key) is None:
         return None
     quants = _quants(qx, _extract_h_quant_params(mods["quant_h_in"]), _extract_h_quant_params(mods["quant_h_out"]))
     if grad:

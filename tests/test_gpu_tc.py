@@ -563,3 +563,39 @@ def test_input_gradient_with_a_zero_weight_row(size):
     ref(xr, h0.double())[0].backward(dout.double())
     layer(xg, h0.cuda())[0].backward(dout.cuda())
     assert rel_err(xg.grad.cpu(), xr.grad) <= PRODUCT_TOL
+
+
+@pytest.mark.parametrize("xbits", [32, 8])
+@pytest.mark.parametrize("grad", [False, True], ids=["infer", "train"])
+def test_layer_call_runs_hooks_and_overridden_quantizers(xbits, grad):
+    """Hooks on the input quantizer (recorded activations) and on the quantizers of unquantised hidden weights fire
+    once per call and their results count; so does a ``forward`` of a subclass or of the instance."""
+    from gru_triton_b200 import quantizers
+    layer = _layer(40, 64, xbits=xbits)
+    cell = layer.cell
+    x, h0 = torch.randn(3, 5, 40, device="cuda"), torch.zeros(5, 64, device="cuda")
+    with torch.set_grad_enabled(grad):
+        plain = layer(x, h0)[0]
+        halved = layer(x * 0.5, h0)[0] if xbits == 32 else None
+        seen = []
+        handles = [m.register_forward_hook(lambda m, a, y: seen.append(y))
+                   for m in (cell.quant_x, cell.quant_W_hr, cell.quant_W_hz, cell.quant_W_hn)]
+        out = layer(x, h0)[0]
+        assert [t.shape for t in seen] == [x.shape] + 3 * [(64, 64)]
+        assert float((out - plain).abs().max()) <= 1e-5
+        for h in handles:
+            h.remove()
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda m, a, y: seen.append(m))
+        layer(x, h0)
+        handle.remove()
+        assert cell.quant_x in seen
+        if xbits == 32:
+            handle = cell.quant_x.register_forward_pre_hook(lambda m, a: (a[0] * 0.5,))
+            assert float((layer(x, h0)[0] - halved).abs().max()) <= 1e-5
+            handle.remove()
+        base = type(cell.quant_x)
+        cell.quant_x.__class__ = type("Doubled", (base,), {"forward": lambda self, v: 2.0 * base.forward(self, v)})
+        doubled = layer(x, h0)[0]
+        cell.quant_x.__class__ = base
+        cell.quant_x.forward = lambda v: 2.0 * base.forward(cell.quant_x, v)
+        assert torch.equal(layer(x, h0)[0], doubled) and not torch.equal(doubled, plain)
