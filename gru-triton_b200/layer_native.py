@@ -226,7 +226,8 @@ def forward(layer, x, h0):
     if type(quant_x) is not Identity:
         if type(quant_x) is FakeQuantizePerTensor and not grad:
             qx = _extract_h_quant_params(quant_x)
-        if qx is None or qx[1] < -127 or qx[2] > 127:
+        # the kernel's grid: int8 codes, a scale whose reciprocal is a normal number (the module takes any, negative ones too)
+        if qx is None or not 1e-30 < qx[0] < 1e30 or qx[1] < -127 or qx[2] > 127:
             qx, x = None, quant_x(x)
             if not _plain_input(x, device):
                 return None

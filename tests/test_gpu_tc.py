@@ -599,3 +599,17 @@ def test_layer_call_runs_hooks_and_overridden_quantizers(xbits, grad):
         cell.quant_x.__class__ = base
         cell.quant_x.forward = lambda v: 2.0 * base.forward(cell.quant_x, v)
         assert torch.equal(layer(x, h0)[0], doubled) and not torch.equal(doubled, plain)
+
+
+@pytest.mark.parametrize("scale", [-0.03, 1e-39, 0.0])
+def test_layer_call_with_an_odd_input_scale(scale, monkeypatch):
+    """A frozen input scale that the conversion kernel has no form of goes through the quantizer module."""
+    from gru_triton_b200 import layer_native
+    layer = _layer(40, 64, xbits=8)
+    layer.cell.quant_x.scale = torch.tensor(scale, device="cuda")
+    x, h0 = torch.randn(3, 5, 40, device="cuda"), torch.zeros(5, 64, device="cuda")
+    with torch.no_grad():
+        native = layer(x, h0)[0]
+        monkeypatch.setattr(layer_native, "forward", lambda *a: None)
+        composed = layer(x, h0)[0]
+    assert torch.allclose(native, composed, rtol=1e-5, atol=1e-5, equal_nan=True)
