@@ -612,6 +612,18 @@ int b200gru_dense_q8_backward(const float* gi, const float* h0, const float* Wq,
                             nullptr, workspace, workspace_bytes_, stream);
 }
 
+int b200gru_test_scan_plan(const b200gru_shape* shape, int backward, int w_codes, const b200gru_quant* q_in, int* plan) {
+  Dims d;
+  if (!parse_shape(shape, &d) || plan == nullptr || (d.kind != B200GRU_DENSE && d.kind != B200GRU_MONARCH)) return B200GRU_INVALID_ARGUMENT;
+  memset(plan, 0, 6 * sizeof(int));
+  if (step_path(d)) { plan[0] = 3; return B200GRU_OK; }
+  const ScanPlan p = plan_scan(d, backward == 0, w_codes != 0, make_quant(q_in));
+  if (!p.found) return B200GRU_UNSUPPORTED;
+  plan[0] = p.tensor ? 2 : 1;
+  if (p.tensor) { plan[1] = p.tc.C; plan[2] = p.tc.N; plan[3] = p.tc.rows; plan[4] = p.tc.clusters; plan[5] = (int)p.tc.smem; }
+  return B200GRU_OK;
+}
+
 void b200gru_test_select_dense_scan(int which) { g_test_choice[2].store(which, std::memory_order_relaxed); }
 
 void b200gru_test_select_gemm(int which) { g_test_choice[3].store(which, std::memory_order_relaxed); }

@@ -862,8 +862,12 @@ __global__ void __launch_bounds__(NT, 1) occupancy_probe_kernel() {}
 
 constexpr size_t STATIC_SMEM = 4096;         // more than any of the kernels declares, and what the system reserves
 
-// Clusters of C CTAs the device holds at once (0: none can be launched) and the shared memory a CTA may ask for.
-struct Device { int active[MAX_C + 1]; size_t smem; };
+// Clusters of C CTAs the device holds at once (0: none can be launched), the shared memory a CTA may ask for, and
+// the least that every launch asks for: half of an SM's.  A CTA takes all 512 columns of tensor memory and then waits
+// for its cluster; a second one on its SM would wait for those columns, and its cluster for it, for good.  Half an
+// SM's memory beside the static part keeps out a second CTA of these kernels and, since they ask for more than
+// that too, one of the tcgen05 products that another stream may run.
+struct Device { int active[MAX_C + 1]; size_t smem, least; };
 static Device device_limits(int C) {
   static std::mutex mu;
   static std::map<int, Device> cache;
@@ -876,9 +880,12 @@ static Device device_limits(int C) {
   if (it == cache.end()) {
     Device d = none;
     for (int c = 0; c <= MAX_C; ++c) d.active[c] = -1;
-    int optin = 0;
+    int optin = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || optin < 65536) return none;
+    if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess) return none;
     d.smem = (size_t)optin - STATIC_SMEM;
+    d.least = (size_t)per_sm / 2;
+    if (d.least > d.smem) return none;
     it = cache.emplace(dev, d).first;
   }
   Device& d = it->second;
@@ -963,7 +970,7 @@ bool choose(bool fwd, int T, int B, int Hb, int nb, bool w_codes, const Quant& q
       found = true;
       *cycles = cost;
       out->C = C; out->N = N; out->rows = rows; out->pw = pw; out->ph = ph; out->clusters = (int)clusters;
-      out->active = active; out->smem = smem;
+      out->active = active; out->smem = smem > dev.least ? smem : dev.least;
     }
   }
   return found;

@@ -613,3 +613,36 @@ def test_layer_call_with_an_odd_input_scale(scale, monkeypatch):
         monkeypatch.setattr(layer_native, "forward", lambda *a: None)
         composed = layer(x, h0)[0]
     assert torch.allclose(native, composed, rtol=1e-5, atol=1e-5, equal_nan=True)
+
+
+def _scan_plan(T, B, H, nb=1, *, backward=False, codes=False, quant=None):
+    """``(kernel, CTAs per cluster, row tile, rows, clusters, shared memory)`` of a dense / block-diagonal scan."""
+    import ctypes
+    from gru_triton_b200 import _lib
+    plan = (ctypes.c_int * 6)()
+    shape = _lib.make_shape("dense" if nb == 1 else "monarch", T, B, H, nb)
+    q = _lib._cquant(quant)
+    assert _lib.load().b200gru_test_scan_plan(ctypes.byref(shape), int(backward), int(codes), ctypes.byref(q), plan) == 0
+    return tuple(plan)
+
+
+def test_one_cluster_scan_cta_per_sm():
+    """A CTA of the tensor-core cluster scan takes all of an SM's tensor memory and waits for its cluster, so no second
+    one may fit beside it: every configuration asks for at least half of the shared memory."""
+    from gru_triton_b200 import _lib
+    per_sm = torch.cuda.get_device_properties(0).shared_memory_per_multiprocessor
+    seen = set()
+    _lib.load().b200gru_test_select_dense_scan(2)
+    try:
+        for H, nb in ((32, 1), (96, 1), (128, 1), (250, 1), (256, 1), (512, 1), (64, 2), (512, 8)):
+            for B in (1, 5, 16, 40, 300):
+                for quant in (None, (0.02, -127, 127)):
+                    for backward in (False, True):
+                        for codes in {False, nb == 1}:
+                            p = _scan_plan(20, B, H, nb, backward=backward, codes=codes, quant=quant)
+                            if p[0] == 2:
+                                seen.add(p[1:3])
+                                assert 2 * p[5] >= per_sm, p
+    finally:
+        _lib.load().b200gru_test_select_dense_scan(0)
+    assert {c for c, _ in seen} >= {1, 3, 4, 8, 16} and {n for _, n in seen} >= {16, 32, 48}
