@@ -85,6 +85,7 @@ SIGNATURES = {
     "b200gru_layer_backward": (_I, [_P, _P, _P, _P]),
     "b200gru_test_select_kernels": (None, [_I, _I]),
     "b200gru_test_scan_plan": (_I, [_SP, _I, _I, _QP, _P]),
+    "b200gru_test_set_scan_status": (_I, [_I]),
     "b200gru_test_select_dense_scan": (None, [_I]),
     "b200gru_test_select_gemm": (None, [_I]),
     "b200gru_test_wait_timeout": (_I, [_P]),

@@ -624,6 +624,8 @@ int b200gru_test_scan_plan(const b200gru_shape* shape, int backward, int w_codes
   return B200GRU_OK;
 }
 
+int b200gru_test_set_scan_status(int value) { return tcc::set_status(value); }
+
 void b200gru_test_select_dense_scan(int which) { g_test_choice[2].store(which, std::memory_order_relaxed); }
 
 void b200gru_test_select_gemm(int which) { g_test_choice[3].store(which, std::memory_order_relaxed); }

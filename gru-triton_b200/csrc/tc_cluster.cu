@@ -108,6 +108,14 @@ __device__ __forceinline__ void bulk_to_peer(uint32_t dst, uint32_t src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
 }
+__device__ __forceinline__ uint32_t load_at_peer(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_at_peer(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void arrive_at_peer(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -118,15 +126,34 @@ __device__ __forceinline__ bool try_wait_cluster(uint32_t bar, uint32_t parity) 
                "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ void wait_cluster(uint32_t bar, uint32_t parity, volatile int* dead, int* status) {
-  if (try_wait_cluster(bar, parity)) return;
+__device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity, volatile int* dead, int* status) {
+  if (try_wait_cluster(bar, parity)) return true;
   const long long start = clock64();
   while (*dead == 0) {
-    if (try_wait_cluster(bar, parity)) return;
+    if (try_wait_cluster(bar, parity)) return true;
     if (clock64() - start > WAIT_BUDGET_CYCLES) {
       *dead = 1;
       atomicExch(status, 1);
     }
+  }
+  return false;
+}
+// Giving up.  A wait that runs out marks its CTA dead, and every later wait of the CTA that would have to wait returns
+// false at once.  Warp 0 turns that into one decision per step: it writes stop[step & 1] before the barrier of all warps,
+// and all of them read it behind that barrier and leave the time loop together (the other parity is not written
+// before everyone has passed the next barrier).  Nothing is issued, committed or copied to a peer on a wait that failed.
+// The end of both kernels: a CTA that gave up tells its whole cluster, and then every CTA of it stays long enough
+// for products and copies in flight to land before any of them leaves.
+__device__ __forceinline__ void leave_together(const cg::cluster_group& cluster, int C, volatile int* dead, int* peer_gave_up) {
+  tc_fence_before();
+  __syncthreads();                     // `dead` is final
+  if (threadIdx.x < C && *dead != 0) store_at_peer(map_to_rank(smem_u32(peer_gave_up), threadIdx.x), 1);
+  cluster.sync();                      // no copy or arrival starts behind this, and none is under way unless somebody gave up
+  if (*reinterpret_cast<volatile int*>(peer_gave_up) != 0) {
+    const long long start = clock64();
+    while (clock64() - start < (1ll << 18)) {
+    }
+    cluster.sync();
   }
 }
 // The 16 compute warps / all 17 warps.
@@ -205,7 +232,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) unsigned long long bar_full[4], bar_empty, bar_acc;
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead;
+  __shared__ int dead, stop[2], peer_gave_up, unhealthy;
   __shared__ float s_wscale[ROWS_A], s_inv_h[MAX_N], s_h[MAX_N];
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -218,7 +245,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   const int nrows = min(a.rows, a.B - b0);
   const int u0 = rank * UNITS;
   const int T = a.T;
-  volatile int* deadp = &dead;
+  volatile int *deadp = &dead, *stopp = stop;
   int* status = a.status;
 
   const uint32_t sent = (uint32_t)(rows8 >> 3) * GROUP;    // bytes of a slab that carry rows
@@ -230,7 +257,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   auto group_bytes = [&](int g) { return (uint32_t)max(0, min(GS, C - g * GS)) * sent; };
 
   if (tid == 0) {
-    dead = 0;
+    dead = stop[0] = stop[1] = peer_gave_up = 0;
+    unhealthy = *reinterpret_cast<volatile int*>(status);
     for (int g = 0; g < 4; ++g) mbar_init(smem_u32(&bar_full[g]), 1);
     mbar_init(smem_u32(&bar_empty), C);
     mbar_init(smem_u32(&bar_acc), 1);
@@ -382,20 +410,22 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   cluster.sync();                      // operands, barriers and tensor memory are ready everywhere
   tc_fence_after();
 
+  // no step where the status word was set when rank 0 started: the cluster leaves as one
+  const int steps = __any_sync(0xffffffffu, load_at_peer(map_to_rank(smem_u32(&unhealthy), 0)) != 0) ? 0 : T;
   if (warp == NW) {
-    // ---- products of a step, a quarter of the slabs at a time as they arrive; one thread waits and issues
+    // ---- products of a step, a quarter of the slabs at a time as they arrive; the warp waits, one lane issues
     const uint64_t dlo = umma_smem_desc(smem_u32(lo), 16, 1024);
     const uint64_t dh = desc_sw64(smem_u32(hbuf), GROUP);
     const uint32_t acc = tmem + TMEM_COLS - NACC * N;
-    for (int t = 0; t < T; ++t) {
-      if (elect_one()) {
+    for (int t = 0; t < steps; ++t) {
+      bool alive = true;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const uint32_t full = smem_u32(&bar_full[g]);
-          if (t > 0) {
-            wait_cluster(full, (t - 1) & 1, deadp, status);
-            if (t + 1 < T) mbar_expect_tx(full, group_bytes(g));
-          }
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t full = smem_u32(&bar_full[g]);
+        if (t > 0) alive = __all_sync(0xffffffffu, wait_cluster(full, (t - 1) & 1, deadp, status));
+        if (!alive) break;
+        if (elect_one()) {
+          if (t > 0 && t + 1 < T) mbar_expect_tx(full, group_bytes(g));
           tc_fence_after();
 #pragma unroll
           for (int s = g * GS; s < (g + 1) * GS; ++s) {
@@ -415,13 +445,17 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
               }
             }
           }
+          if (g == 3) {
+            umma_commit(smem_u32(&bar_acc));
+            if (t + 1 < T) umma_commit_cluster(smem_u32(&bar_empty), (uint16_t)((1u << C) - 1));
+          }
         }
-        umma_commit(smem_u32(&bar_acc));
-        if (t + 1 < T) umma_commit_cluster(smem_u32(&bar_empty), (uint16_t)((1u << C) - 1));
+        __syncwarp();
       }
       __syncwarp();
       if (t + 1 < T) {
         bar_all();                                         // the new slab is staged: one copy to every peer
+        if (__any_sync(0xffffffffu, stopp[t & 1] != 0)) break;
         if (lane < C) {
           const uint32_t peer = (uint32_t)(rank + lane < C ? rank + lane : rank + lane - C);
           bulk_to_peer(map_to_rank(smem_u32(hbuf) + (uint32_t)lane * SLAB, peer), smem_u32(stg), sent,
@@ -438,7 +472,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
     float sh[RPW];
 #pragma unroll
     for (int i = 0; i < RPW; ++i) sh[i] = (PH == 2) ? s_h[warp + i * NW] : 1.f;
-    for (int t = 0; t < T; ++t) {
+    for (int t = 0; t < steps; ++t) {
       float ngr[RPW], ngz[RPW], ngn[RPW];
 #pragma unroll
       for (int i = 0; i < RPW; ++i) {
@@ -448,7 +482,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
           ngr[i] = __ldcs(g); ngz[i] = __ldcs(g + H); ngn[i] = __ldcs(g + 2 * H);
         }
       }
-      mbar_wait(smem_u32(&bar_acc), t & 1, deadp, status);
+      bool alive = mbar_wait(smem_u32(&bar_acc), t & 1, deadp, status);
       __syncwarp();
       tc_fence_after();
       if (q < 3) {
@@ -488,7 +522,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
       }
       if (t + 1 < T) {
         // every peer has finished reading h_{t-1} (and so has received the slab this buffer held)
-        wait_cluster(smem_u32(&bar_empty), t & 1, deadp, status);
+        alive = wait_cluster(smem_u32(&bar_empty), t & 1, deadp, status) && alive;
+        if (warp == 0 && !alive) stopp[t & 1] = 1;
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < RPW; ++i) {
@@ -508,6 +543,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
         }
         fence_async_smem();
         bar_all();
+        if (__any_sync(0xffffffffu, stopp[t & 1] != 0)) break;
       }
 #pragma unroll
       for (int i = 0; i < RPW; ++i) {
@@ -525,8 +561,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
       }
     }
   }
-  tc_fence_before();
-  cluster.sync();                      // nobody leaves while a peer's copy or arrival may be under way
+  leave_together(cluster, C, deadp, &peer_gave_up);
   if (warp == NW) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -547,7 +582,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) unsigned long long bar_recv, bar_empty, bar_acc[4];
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead;
+  __shared__ int dead, stop[2], peer_gave_up, unhealthy;
   __shared__ float s_fold[ROWS_A], s_scale[ROWS_A];
   __shared__ __align__(16) float s_inv[2][4 * NW];          // inverse row scales of dgh, by step parity
 
@@ -562,7 +597,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   const int RG = (a.rows + 3) >> 2;                        // groups of four rows that are exchanged
   const int u0 = rank * UNITS;
   const int T = a.T;
-  volatile int* deadp = &dead;
+  volatile int *deadp = &dead, *stopp = stop;
   int* status = a.status;
   const uint32_t recv_bytes = (uint32_t)(C * RG * 512);
 
@@ -572,7 +607,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   float* stage = recv + (size_t)C * RG * 128;              // [destination][row group][unit][4 rows]
 
   if (tid == 0) {
-    dead = 0;
+    dead = stop[0] = stop[1] = peer_gave_up = 0;
+    unhealthy = *reinterpret_cast<volatile int*>(status);
     mbar_init(smem_u32(&bar_recv), 1);
     mbar_init(smem_u32(&bar_empty), C);
     for (int m = 0; m < 4; ++m) mbar_init(smem_u32(&bar_acc[m]), 1);
@@ -687,11 +723,14 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   cluster.sync();
   tc_fence_after();
 
+  // nothing is done where the status word was set when rank 0 started: the cluster leaves as one
+  const int last = __any_sync(0xffffffffu, load_at_peer(map_to_rank(smem_u32(&unhealthy), 0)) != 0) ? -1 : T;
   if (warp == NW) {
     const uint64_t db0 = desc_sw64(smem_u32(bop), 512);
     const uint64_t da0 = desc_sw64(smem_u32(lo), 512);
-    for (int it = 0; it < T; ++it) {
+    for (int it = 0; it < last; ++it) {
       bar_all();                                           // dgh of this step is in place
+      if (__any_sync(0xffffffffu, stopp[it & 1] != 0)) break;
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
@@ -715,15 +754,15 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
       __syncwarp();
     }
   } else {
-    for (int it = 0; it <= T; ++it) {
+    bool alive = true;                                     // every wait of this warp so far
+    for (int it = 0; it <= last; ++it) {
       const int t = T - 1 - it;
       float dh[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) dh[i] = 0.f;
       if (it > 0) {
-        wait_cluster(smem_u32(&bar_recv), (it - 1) & 1, deadp, status);
-        __syncwarp();
-        if (tid == 0 && it < T) mbar_expect_tx(smem_u32(&bar_recv), recv_bytes);
+        alive = __all_sync(0xffffffffu, wait_cluster(smem_u32(&bar_recv), (it - 1) & 1, deadp, status)) && alive;
+        if (tid == 0 && it < T && alive) mbar_expect_tx(smem_u32(&bar_recv), recv_bytes);
         // scalar reads of [unit][4 rows]: the rows of a unit are rotated by unit / 8, so that the 32 units of a row
         // lie in 32 banks
 #pragma unroll
@@ -747,8 +786,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
       float gr[R], gz[R], gn[R];
       // the products of the previous step have read the operand (this rank's partial sums may be
       // complete while the last tiles are still under way)
-      if (it > 0) mbar_wait(smem_u32(&bar_acc[TILES - 1]), (it - 1) & 1, deadp, status);
-      __syncwarp();
+      if (it > 0) alive = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc[TILES - 1]), (it - 1) & 1, deadp, status)) && alive;
+      if (tid == 0 && !alive) stopp[it & 1] = 1;
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         // entries beyond the batch run on zeros, so that the rows of a thread interleave
@@ -781,15 +820,17 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
       fetch(t - 1);
       fence_async_smem();
       bar_all();
+      if (__any_sync(0xffffffffu, stopp[it & 1] != 0)) break;
       // the partial sums of the previous step have been read: peers may overwrite them
       if (it > 0 && warp < C && lane == 0) arrive_at_peer(map_to_rank(smem_u32(&bar_empty), (uint32_t)warp));
       __syncwarp();
       // ---- partial sums of 32 positions to the rank that owns them
       const int dest = m_own * 4 + q_own;
       if (dest < C) {
-        mbar_wait(smem_u32(&bar_acc[m_own]), it & 1, deadp, status);
-        if (it > 0) wait_cluster(smem_u32(&bar_empty), (it - 1) & 1, deadp, status);
-        __syncwarp();
+        bool ready = mbar_wait(smem_u32(&bar_acc[m_own]), it & 1, deadp, status);
+        if (it > 0) ready = wait_cluster(smem_u32(&bar_empty), (it - 1) & 1, deadp, status) && ready;
+        ready = __all_sync(0xffffffffu, ready);
+        alive = alive && ready;
         tc_fence_after();
         const uint32_t ts = acc + ((uint32_t)(q_own * 32) << 16) + (uint32_t)(m_own * N);
         const int rot = lane >> 3;
@@ -806,7 +847,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
         tc_fence_before();
         fence_async_smem();
         __syncwarp();
-        if (lane == 0)
+        if (lane == 0 && ready)
           bulk_to_peer(map_to_rank(smem_u32(recv) + (uint32_t)(rank * RG * 512), (uint32_t)dest),
                        smem_u32(stage + (size_t)dest * RG * 128), (uint32_t)(RG * 512),
                        map_to_rank(smem_u32(&bar_recv), (uint32_t)dest));
@@ -821,8 +862,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
         }
     }
   }
-  tc_fence_before();
-  cluster.sync();
+  leave_together(cluster, C, deadp, &peer_gave_up);
   if (warp == NW) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -1007,6 +1047,8 @@ int launch(bool fwd, const Config& c, Args a, cudaStream_t st) {
   note_launch();
   return check_launch(fwd ? "tcc_fwd_kernel" : "tcc_bwd_kernel");
 }
+
+int set_status(int value) { return cudaMemcpyToSymbol(g_tcc_status, &value, sizeof(int)) == cudaSuccess ? B200GRU_OK : B200GRU_LAUNCH_FAILURE; }
 
 int read_status(int reset) {
   int v = 0;

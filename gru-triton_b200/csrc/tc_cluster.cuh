@@ -41,6 +41,7 @@ struct Config {
 bool choose(bool fwd, int T, int B, int Hb, int nb, bool w_codes, const Quant& qin, Config* out, double* cycles);
 int launch(bool fwd, const Config& c, Args a, cudaStream_t st);
 int read_status(int reset);
+int set_status(int value);              // tests only
 
 }  // namespace tcc
 }  // namespace b200gru

@@ -332,11 +332,13 @@ int b200gru_calibration_scan(const b200gru_shape* shape, const float* gi, const 
  * choice by shape.
  * b200gru_test_scan_plan: the kernel of a dense / block-diagonal scan as plan[0] (1 FP32 clusters, 2 tensor-core clusters,
  * 3 one product per step); for 2 its CTAs per cluster, row tile, rows per cluster, clusters and dynamic shared memory.
+ * b200gru_test_set_scan_status: writes the status word of the tensor-core cluster scans, as a wait that ran out would.
  * b200gru_test_wait_timeout: launches one tiny kernel whose bounded wait must run out (it waits
  * about a millisecond for bytes nothing sends), which sets the flag b200gru_device_status
  * reports; the kernel returns normally and the device stays usable. */
 void b200gru_test_select_kernels(int butterfly_register_kernels, int diagonal_register_ring);
 int b200gru_test_scan_plan(const b200gru_shape* shape, int backward, int w_codes, const b200gru_quant* q_in, int* plan);
+int b200gru_test_set_scan_status(int value);
 void b200gru_test_select_dense_scan(int which);
 void b200gru_test_select_gemm(int which);
 int b200gru_test_wait_timeout(void* stream);

@@ -646,3 +646,37 @@ def test_one_cluster_scan_cta_per_sm():
     finally:
         _lib.load().b200gru_test_select_dense_scan(0)
     assert {c for c, _ in seen} >= {1, 3, 4, 8, 16} and {n for _, n in seen} >= {16, 32, 48}
+
+
+@pytest.mark.parametrize("B,H", [(3, 32), (5, 96), (40, 512)])
+def test_zz_cluster_scan_leaves_when_the_status_word_is_set(B, H):
+    """A cluster that starts while the status word is set leaves as one, forward and backward: nothing is written, the
+    word is reported, and once it is cleared the same call gives the same bits as before."""
+    from gru_triton_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(H)
+    T = 30
+    gi, h0, dout = (torch.randn(s, device="cuda", generator=g) for s in ((T, B, 3 * H), (B, H), (T, B, H)))
+    W, bh = torch.randn(3 * H, H, device="cuda", generator=g) * 0.04, torch.zeros(3 * H, device="cuda")
+    lib.b200gru_test_select_dense_scan(2)
+    try:
+        out, save = _lib.scan_forward("dense", gi, h0, W, bh, None, None, want_save=True)
+        dgi = _lib.scan_backward("dense", gi, h0, W, bh, out, dout, save, None, None)[0]
+        torch.cuda.synchronize()
+        assert lib.b200gru_test_set_scan_status(1) == 0
+        # blocks of the allocator that a finished call gave back: outputs nobody writes keep what lay there
+        marked, ws = torch.full_like(out, 7.0), torch.empty(1 << 24, device="cuda", dtype=torch.uint8)
+        q = _lib._cquant(None)
+        assert lib.b200gru_dense_forward(gi.data_ptr(), h0.data_ptr(), W.data_ptr(), bh.data_ptr(), T, B, H, q, q, marked.data_ptr(),
+                                         None, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream) == 0
+        _lib.scan_backward("dense", gi, h0, W, bh, out, dout, save, None, None)
+        torch.cuda.synchronize()
+        assert bool((marked == 7.0).all())
+        with pytest.raises(_lib.DeviceWaitTimeout):
+            _lib.check_device_status(reset=True)
+        again, save = _lib.scan_forward("dense", gi, h0, W, bh, None, None, want_save=True)
+        dgi2 = _lib.scan_backward("dense", gi, h0, W, bh, again, dout, save, None, None)[0]
+        assert torch.equal(again, out) and torch.equal(dgi2, dgi)
+    finally:
+        lib.b200gru_test_set_scan_status(0)
+        lib.b200gru_test_select_dense_scan(0)
