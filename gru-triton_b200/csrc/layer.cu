@@ -421,6 +421,7 @@ int b200gru_layer_backward(const int* dims, const float* quants, const void* con
   Layer L;
   Kept k;
   if (!parse(dims, &L)) return B200GRU_INVALID_ARGUMENT;
+  const bool scan = L.flags != B200GRU_LAYER_PROJECTION, projection = L.flags != B200GRU_LAYER_SCAN;
   const float* x = static_cast<const float*>(ptrs[0]);
   const float* h0 = static_cast<const float*>(ptrs[1]);
   const float* out = static_cast<const float*>(ptrs[2]);
@@ -429,21 +430,24 @@ int b200gru_layer_backward(const int* dims, const float* quants, const void* con
   char* kept = static_cast<char*>(const_cast<void*>(ptrs[5]));
   char* scratch = static_cast<char*>(const_cast<void*>(ptrs[6]));
   float* const* o = reinterpret_cast<float* const*>(const_cast<void* const*>(ptrs)) + 7;   // dx, dh0, dWi, dWh, dbi, dbh, dgi
-  if (!x || !h0 || !out || !dout || !save || !kept || !scratch || !o[1] || !o[3] || !o[5] || !o[6]) return B200GRU_INVALID_ARGUMENT;
+  if (!kept || !scratch || !o[6]) return B200GRU_INVALID_ARGUMENT;
+  if (scan && (!h0 || !out || !dout || !save || !o[1] || !o[3] || !o[5])) return B200GRU_INVALID_ARGUMENT;
+  if (projection && !x) return B200GRU_INVALID_ARGUMENT;
   carve(L, kept, &k);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const b200gru_quant qi = quant_of(quants + 4), qo = quant_of(quants + 8);
   float* dgi = o[6];
   float* dWq = nullptr;
   if (L.bits_h <= 8) { dWq = reinterpret_cast<float*>(scratch); scratch += pad(L.w_elems * 4); }
-  int rc;                               // gi is read only where the gates were not saved; dgi stands in for it
-  const bool q8 = L.bits_h <= 8, gi_in = keeps_gi(L);
-  rc = layer_scan_backward(&L.shape, gi_in ? save : dgi, h0, q8 ? k.Wh_q : k.Wh, k.Wh_codes, q8 ? k.Wh_scale : nullptr, k.b_h, out, dout,
-                           gi_in ? nullptr : save, &qi, &qo, dgi, o[1], q8 ? dWq : o[3], o[5], o[4], scratch,
-                           scan_ws(L, gi_in ? 1 : 2), stream);
-  if (!rc && q8) rc = launch_quantize_rows_backward(k.Wh, dWq, 3 * L.H, L.H, L.bits_h, o[3], st);
-  if (rc) return rc;
-  return linear_backward(L, k, x, dgi, o[2], o[0], scratch, st);
+  if (scan) {                           // gi is read only where the gates were not saved; dgi stands in for it
+    const bool q8 = L.bits_h <= 8, gi_in = keeps_gi(L);
+    int rc = layer_scan_backward(&L.shape, gi_in ? save : dgi, h0, q8 ? k.Wh_q : k.Wh, k.Wh_codes, q8 ? k.Wh_scale : nullptr, k.b_h, out,
+                                 dout, gi_in ? nullptr : save, &qi, &qo, dgi, o[1], q8 ? dWq : o[3], o[5], o[4], scratch,
+                                 scan_ws(L, gi_in ? 1 : 2), stream);
+    if (!rc && q8) rc = launch_quantize_rows_backward(k.Wh, dWq, 3 * L.H, L.H, L.bits_h, o[3], st);
+    if (rc) return rc;
+  }
+  return projection ? linear_backward(L, k, x, dgi, o[2], o[0], scratch, st) : B200GRU_OK;
 }
 
 }  // extern "C"

@@ -31,10 +31,11 @@ _INPUT_QUANTIZERS = (Identity, FakeQuantizePerTensor, FakeQuantizePerChannel, Fa
 
 @lru_cache(maxsize=512)
 def _plan(kind, T, B, I, H, nblocks, log2_hpad, bits_i, bits_h):
-    """``(dims, kept bytes, forward scratch, backward scratch)`` of a shape, or None if it has none."""
-    dims = _INTS(_lib.KIND[kind], T, B, I, H, nblocks, log2_hpad, bits_i, bits_h, 0)
+    """``((dims, of the scan's backward, of the projection's), kept bytes, forward scratch, backward scratch)`` of a
+    shape, or None if it has none."""
+    dims = [_INTS(_lib.KIND[kind], T, B, I, H, nblocks, log2_hpad, bits_i, bits_h, part) for part in range(3)]
     sizes = _SIZES()
-    if _lib.load().b200gru_layer_sizes(dims, sizes):
+    if _lib.load().b200gru_layer_sizes(dims[0], sizes):
         return None
     return (dims, *sizes)
 
@@ -79,7 +80,7 @@ def _transformed() -> bool:
 
 
 def _parameters(cell, kind, device, I, H):
-    """``(params, nblocks, log2_hpad)``: input weights, hidden weights, input biases, hidden biases per gate."""
+    """``(params, nblocks, log2_hpad)``: input weights, hidden weights, input biases, hidden biases per gate (no biases: six)."""
     own, mods = cell._parameters, cell._modules
     wi = [own.get("W_i" + g) for g in _GATES]
     nblocks, log2_hpad = 1, 0
@@ -120,8 +121,8 @@ def _addresses(params):
 
 
 def _run(x, h0, key, quants, params, train):
-    plan = _plan(*key)
-    dims, kept_bytes, scratch_bytes, _ = plan
+    """``(out, save, kept, gi)`` of a whole forward call."""
+    dims, kept_bytes, scratch_bytes, _ = _plan(*key)
     kind, T, B, I, H = key[:5]
     device = x.device
     out = torch.empty((T, B, H), device=device, dtype=torch.float32)
@@ -132,11 +133,11 @@ def _run(x, h0, key, quants, params, train):
     scratch = torch.empty(scratch_bytes, device=device, dtype=torch.uint8)
     ptrs = _FWD_PTRS(x.data_ptr(), h0.data_ptr(), *_addresses(params), out.data_ptr(), None if save is None else save.data_ptr(),
                      kept.data_ptr(), scratch.data_ptr(), gi.data_ptr())
-    rc = _call(_lib.load().b200gru_layer_forward, dims, quants, ptrs, device)
+    rc = _call(_lib.load().b200gru_layer_forward, dims[0], quants, ptrs, device)
     if rc:
         _lib._raise(rc, f"{kind} layer forward")
     _lib._after_call()
-    return out, (gi if kind == "diagonal" else save), kept
+    return out, save, kept, gi
 
 
 def _call(fn, dims, quants, ptrs, device):
@@ -147,31 +148,72 @@ def _call(fn, dims, quants, ptrs, device):
         return fn(dims, quants, ptrs, torch._C._cuda_getCurrentRawStream(index))
 
 
-class LayerFunction(torch.autograd.Function):
-    """``out[T,B,H]`` of a layer call; ``params`` as :func:`_parameters` lists them."""
+def _restored(ctx, dtypes):
+    """Saved tensors in the form the library reads: saved-tensor hooks may hand back another dtype or layout."""
+    device = ctx.device
+    return [t if t.dtype is dtype and t.device == device and t.is_contiguous() else t.to(device, dtype).contiguous()
+            for t, dtype in zip(ctx.saved_tensors, dtypes)]
+
+
+# One library call runs the whole forward, but two autograd nodes stand for it, the projection's and the scan's:
+# the gradients of the hidden side are complete, and their reduction can start, before the projection's backward runs.
+# Both biases belong to the scan's node, whose kernels sum them from one read of dgi.
+
+class ProjectionFunction(torch.autograd.Function):
+    """``gi[T,B,3H]``; runs the scan as well and leaves ``(out, save, kept)`` in ``call``, which holds what it needs beside x."""
 
     @staticmethod
-    def forward(ctx, x, h0, key, quants, *params):
-        train = any(ctx.needs_input_grad)
-        out, save, kept = _run(x, h0, key, quants, params, train)
-        ctx.key, ctx.quants, ctx.nparams = key, quants, len(params)
-        if train:
-            ctx.save_for_backward(x, h0, out, save, kept)
+    def forward(ctx, x, key, quants, call, *wi):
+        h0, params = call
+        out, save, kept, gi = _run(x, h0, key, quants, params, True)
+        call[:] = out, save, kept
+        ctx.key, ctx.quants, ctx.device = key, quants, x.device
+        if any(ctx.needs_input_grad):
+            ctx.save_for_backward(x, kept)
+        return gi
+
+    @staticmethod
+    def backward(ctx, dgi):
+        x, kept = _restored(ctx, (torch.float32, torch.uint8))
+        need = ctx.needs_input_grad
+        kind, T, B, I, H = ctx.key[:5]
+        dims, _, _, scratch_bytes = _plan(*ctx.key)
+        device = ctx.device
+        dgi = dgi.contiguous()
+        dx = torch.empty_like(x) if need[0] else None
+        dwi = torch.empty((3, H, I), device=device, dtype=torch.float32) if any(need[4:]) else None
+        scratch = torch.empty(scratch_bytes, device=device, dtype=torch.uint8)
+        ptrs = _BWD_PTRS(x.data_ptr(), None, None, None, None, kept.data_ptr(), scratch.data_ptr(), None if dx is None else dx.data_ptr(),
+                         None, None if dwi is None else dwi.data_ptr(), None, None, None, dgi.data_ptr())
+        rc = _call(_lib.load().b200gru_layer_backward, dims[2], ctx.quants, ptrs, device)
+        if rc:
+            _lib._raise(rc, f"{kind} layer backward")
+        _lib._after_call()
+        grads = dwi.unbind(0) if dwi is not None else (None, None, None)
+        return (dx, None, None, None, *(g if n else None for g, n in zip(grads, need[4:])))
+
+
+class ScanFunction(torch.autograd.Function):
+    """``out[T,B,H]`` that the projection's call left in ``call``; ``params``: hidden weights, then (if any) both biases."""
+
+    @staticmethod
+    def forward(ctx, gi, h0, key, quants, call, *params):
+        out, save, kept = call
+        ctx.key, ctx.quants, ctx.nparams, ctx.device = key, quants, len(params), gi.device
+        ctx.save_for_backward(h0, out, gi if save is None else save, kept)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        x, h0, out, save, kept = ctx.saved_tensors
+        h0, out, save, kept = _restored(ctx, (torch.float32, torch.float32, torch.float32, torch.uint8))
         need = ctx.needs_input_grad
         kind, T, B, I, H, nblocks, log2_hpad = ctx.key[:7]
-        has_bias = ctx.nparams == 12
-        want_dx, want_wi, want_bi = need[0], any(need[4:7]), has_bias and any(need[10:13])
+        has_bias = ctx.nparams == 9
+        want_bi = has_bias and any(need[8:11])
         dims, _, _, scratch_bytes = _plan(*ctx.key)
-        device = x.device
+        device = ctx.device
         dout = dout.contiguous()
-        dx = torch.empty_like(x) if want_dx else None
         dh0 = torch.empty_like(h0)
-        dwi = torch.empty((3, H, I), device=device, dtype=torch.float32) if want_wi else None
         shape = {"dense": (H, H), "diagonal": (H,), "monarch": (nblocks, H // nblocks, H // nblocks),
                  "butterfly": (1, nblocks, log2_hpad, (1 << log2_hpad) // 2, 2, 2)}[kind]
         dwh = torch.empty((3, *shape), device=device, dtype=torch.float32)
@@ -179,17 +221,15 @@ class LayerFunction(torch.autograd.Function):
         dbh = torch.empty((3, H), device=device, dtype=torch.float32)
         dgi = torch.empty((T, B, 3 * H), device=device, dtype=torch.float32)
         scratch = torch.empty(scratch_bytes, device=device, dtype=torch.uint8)
-        ptrs = _BWD_PTRS(x.data_ptr(), h0.data_ptr(), out.data_ptr(), dout.data_ptr(), save.data_ptr(), kept.data_ptr(),
-                         scratch.data_ptr(), dx.data_ptr() if want_dx else None, dh0.data_ptr(),
-                         dwi.data_ptr() if want_wi else None, dwh.data_ptr(), dbi.data_ptr() if want_bi else None, dbh.data_ptr(), dgi.data_ptr())
-        rc = _call(_lib.load().b200gru_layer_backward, dims, ctx.quants, ptrs, device)
+        ptrs = _BWD_PTRS(None, h0.data_ptr(), out.data_ptr(), dout.data_ptr(), save.data_ptr(), kept.data_ptr(), scratch.data_ptr(),
+                         None, dh0.data_ptr(), None, dwh.data_ptr(), dbi.data_ptr() if want_bi else None, dbh.data_ptr(), dgi.data_ptr())
+        rc = _call(_lib.load().b200gru_layer_backward, dims[1], ctx.quants, ptrs, device)
         if rc:
             _lib._raise(rc, f"{kind} layer backward")
         _lib._after_call()
-        none = (None, None, None)
-        grads = [dx, dh0, None, None, *(dwi.unbind(0) if want_wi else none), *dwh.unbind(0)]
+        grads = [dgi, dh0, None, None, None, *dwh.unbind(0)]
         if has_bias:
-            grads += [*(dbi.unbind(0) if want_bi else none), *dbh.unbind(0)]
+            grads += [*(dbi.unbind(0) if want_bi else (None, None, None)), *dbh.unbind(0)]
         return tuple(g if n else None for g, n in zip(grads, need))
 
 
@@ -236,7 +276,9 @@ def forward(layer, x, h0):
         return None
     quants = _quants(qx, _extract_h_quant_params(mods["quant_h_in"]), _extract_h_quant_params(mods["quant_h_out"]))
     if grad:
-        return LayerFunction.apply(x, h0, key, quants, *params)
+        call = [h0, params]
+        gi = ProjectionFunction.apply(x, key, quants, call, *params[:3])
+        return ScanFunction.apply(gi, h0, key, quants, call, *params[3:])
     return _run(x, h0, key, quants, params, False)[0]
 
 

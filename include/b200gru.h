@@ -257,15 +257,17 @@ int b200gru_column_sums(const float* src, size_t rows, int cols, float* dst, voi
  * Stands in for GRULayer._forward_fast_dispatch (src/gru_qat/gru_layer.py:234-302) and its autograd.
  *   dims   {kind, T, B, I, H, nblocks, log2_hpad, weight bits of the input side, of the hidden side (dense), flags};
  *          I and H multiples of 8; bits 32 (none) or 2..8 (per output row, symmetric, dynamic scale);
- *          0 (reserved)
+ *          0, or which half of the backward to run: the scan's, or the projection's from dgi
  *   quants {scale, qmin, qmax, enabled} of the input, fq_in and fq_out (frozen); the input one only where no backward follows
  *   sizes  bytes of the buffers {kept, forward scratch, backward scratch}, 256-byte aligned
  *   forward ptrs   {x[T][B][I], h0[B][H], Wi r,z,n, Wh r,z,n, bi r,z,n, bh r,z,n (biases may be NULL), out[T][B][H],
  *                   save ([4][T][B][H] where a backward call follows, else NULL; diagonal: NULL), kept, scratch,
  *                   gi[T][B][3H] (scratch; a diagonal backward reads it)}
  *   backward ptrs  {x, h0, out, dout, save (diagonal: gi), kept, scratch, dx or NULL, dh0, dWi[3H][I] or NULL, dWh,
- *                   dbi[3H] or NULL, dbh[3H], dgi[T][B][3H] (scratch)}
+ *                   dbi[3H] or NULL, dbh[3H], dgi[T][B][3H] (written by the scan's half, read by the projection's)};
+ *                  the scan's half takes x, dx and dWi as NULL, the projection's all but x, kept, scratch, dx, dWi, dgi
  * Hidden weights per gate: [H][H], [H], [nblocks][H/nblocks][H/nblocks] or [nblocks][log2_hpad][2^log2_hpad / 2][2][2]. */
+enum { B200GRU_LAYER_SCAN = 1, B200GRU_LAYER_PROJECTION = 2 };
 int b200gru_layer_sizes(const int* dims, size_t* sizes);
 int b200gru_layer_forward(const int* dims, const float* quants, const void* const* ptrs, void* stream);
 int b200gru_layer_backward(const int* dims, const float* quants, const void* const* ptrs, void* stream);

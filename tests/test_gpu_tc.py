@@ -680,3 +680,38 @@ def test_zz_cluster_scan_leaves_when_the_status_word_is_set(B, H):
     finally:
         lib.b200gru_test_set_scan_status(0)
         lib.b200gru_test_select_dense_scan(0)
+
+
+@pytest.mark.parametrize("kind", [None, "diagonal", "monarch", "butterfly"])
+def test_hidden_gradients_are_ready_before_the_projection_backward(kind):
+    """What ``OverlappedReducer`` overlaps: the last hidden gradient is accumulated, and its hook runs, before the
+    kernels of the projection's backward are launched."""
+    from gru_triton_b200 import _lib
+    from gru_triton_b200.data_parallel import hidden_then_input_buckets
+    layer = _layer(40, 64, kind=kind)
+    hidden, rest = hidden_then_input_buckets(layer)
+    at = {}
+    for p in hidden + rest:
+        p.register_post_accumulate_grad_hook(lambda p: at.__setitem__(p, _lib.load().b200gru_launch_count()))
+    layer(torch.randn(6, 5, 40, device="cuda", requires_grad=True), torch.zeros(5, 64, device="cuda"))[0].sum().backward()
+    weights = [p for n, p in layer.named_parameters() if ".W_i" in n]
+    assert len(at) == len(hidden) + len(rest) and max(at[p] for p in hidden) < min(at[p] for p in weights)
+
+
+@pytest.mark.parametrize("kind,wbits", [(None, 32), (None, 8), ("diagonal", 32)])
+def test_layer_backward_under_saved_tensor_hooks(kind, wbits):
+    """Saved tensors that come back as others: on the host, widened, or not contiguous."""
+    layer = _layer(40, 64, kind=kind, wbits=wbits)
+    x, h0 = torch.randn(6, 5, 40, device="cuda"), torch.zeros(5, 64, device="cuda")
+    def grads(pack, unpack):
+        layer.zero_grad(set_to_none=True)
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            out = layer(x, h0)[0]
+        out.square().sum().backward()
+        return [p.grad for p in layer.parameters()]
+    plain = grads(lambda t: t, lambda t: t)
+    back = lambda t: t.double()
+    apart = lambda t: torch.stack([t, t], -1)[..., 0]
+    for pack, unpack in ((lambda t: t.cpu(), lambda t: t.cuda()), (back, lambda t: t), (lambda t: t, apart)):
+        for a, b in zip(plain, grads(pack, unpack)):
+            assert torch.equal(a, b)
