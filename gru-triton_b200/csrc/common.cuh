@@ -122,12 +122,12 @@ __device__ __forceinline__ float ste_mask(float x, const Quant& q) {
 }
 
 // Power of two s with mx * s in [2^14, 2^15) and its inverse, both normal numbers; 1 and 1 for infinities and NaN.  A
-// zero row has s = 1 and inverse 0: the backward products fold the inverse scales of the weight rows into the
-// gradient before that takes a scale of its own, and a row that contributes nothing must not set its largest entry
-// (with factor 1 against 2^-28 for live rows of 1e-4 it pushed those into the fp16 subnormals).
+// zero row has s = 1 and the smallest normal number as its "inverse": the backward products fold the inverse scales of the
+// weight rows into the gradient before that takes a scale of its own, and a row that contributes nothing must not set
+// its largest entry (with factor 1 against 2^-28 for live rows of 1e-4 it pushed those into the fp16 subnormals).
 __device__ __forceinline__ void pow2_row_scale(float mx, float* s, float* inv) {
   int e = (int)((__float_as_uint(mx) >> 23) & 0xffu) - 127;       // floor(log2 mx)
-  if (!(mx > 0.f) || e > 127) { *s = 1.f; *inv = mx == 0.f ? 0.f : 1.f; return; }
+  if (!(mx > 0.f) || e > 127) { *s = 1.f; *inv = mx == 0.f ? 1.1754943508222875e-38f : 1.f; return; }
   e = 14 - max(-100, e);
   *s = __uint_as_float((uint32_t)(127 + e) << 23);
   *inv = __uint_as_float((uint32_t)(127 - e) << 23);
