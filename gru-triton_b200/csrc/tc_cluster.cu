@@ -139,9 +139,9 @@ __device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity, vola
   return false;
 }
 // Giving up.  A wait that runs out marks its CTA dead, and every later wait of the CTA that would have to wait returns
-// false at once.  Warp 0 turns that into one decision per step: it writes stop[step & 1] before the barrier of all warps,
-// and all of them read it behind that barrier and leave the time loop together (the other parity is not written
-// before everyone has passed the next barrier).  Nothing is issued, committed or copied to a peer on a wait that failed.
+// false at once.  The barrier of all warps in every step carries that along (bar_all_any): all warps learn of it at the same
+// point and leave the time loop together.  Nothing is committed or copied to a peer, and no byte expected, on a wait that
+// failed.  (Products may be issued: they read and write this CTA's own memory.)
 // The end of both kernels: a CTA that gave up tells its whole cluster, and then every CTA of it stays long enough
 // for products and copies in flight to land before any of them leaves.
 __device__ __forceinline__ void leave_together(const cg::cluster_group& cluster, int C, volatile int* dead, int* peer_gave_up) {
@@ -158,7 +158,12 @@ __device__ __forceinline__ void leave_together(const cg::cluster_group& cluster,
 }
 // The 16 compute warps / all 17 warps.
 __device__ __forceinline__ void bar_compute() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); }
-__device__ __forceinline__ void bar_all() { asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory"); }
+__device__ __forceinline__ bool bar_all_any(bool gave_up) {       // whether any thread of the CTA gave up
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 2, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(any) : "r"((uint32_t)gave_up), "n"(NT) : "memory");
+  return __any_sync(0xffffffffu, any != 0);                // (a vote, so that the compiler knows the warp stays together)
+}
 
 __device__ __forceinline__ float warp_max(float v) {              // v >= 0 (or NaN, which counts as largest)
   return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
@@ -232,7 +237,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) unsigned long long bar_full[4], bar_empty, bar_acc;
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead, stop[2], peer_gave_up, unhealthy;
+  __shared__ int dead, peer_gave_up, unhealthy;
   __shared__ float s_wscale[ROWS_A], s_inv_h[MAX_N], s_h[MAX_N];
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -245,7 +250,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   const int nrows = min(a.rows, a.B - b0);
   const int u0 = rank * UNITS;
   const int T = a.T;
-  volatile int *deadp = &dead, *stopp = stop;
+  volatile int* deadp = &dead;
   int* status = a.status;
 
   const uint32_t sent = (uint32_t)(rows8 >> 3) * GROUP;    // bytes of a slab that carry rows
@@ -257,7 +262,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   auto group_bytes = [&](int g) { return (uint32_t)max(0, min(GS, C - g * GS)) * sent; };
 
   if (tid == 0) {
-    dead = stop[0] = stop[1] = peer_gave_up = 0;
+    dead = peer_gave_up = 0;
     unhealthy = *reinterpret_cast<volatile int*>(status);
     for (int g = 0; g < 4; ++g) mbar_init(smem_u32(&bar_full[g]), 1);
     mbar_init(smem_u32(&bar_empty), C);
@@ -413,19 +418,20 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   // no step where the status word was set when rank 0 started: the cluster leaves as one
   const int steps = __any_sync(0xffffffffu, load_at_peer(map_to_rank(smem_u32(&unhealthy), 0)) != 0) ? 0 : T;
   if (warp == NW) {
-    // ---- products of a step, a quarter of the slabs at a time as they arrive; the warp waits, one lane issues
+    // ---- products of a step, a quarter of the slabs at a time as they arrive; one lane waits and issues
     const uint64_t dlo = umma_smem_desc(smem_u32(lo), 16, 1024);
     const uint64_t dh = desc_sw64(smem_u32(hbuf), GROUP);
     const uint32_t acc = tmem + TMEM_COLS - NACC * N;
     for (int t = 0; t < steps; ++t) {
-      bool alive = true;
+      bool ok = true;
+      if (elect_one()) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const uint32_t full = smem_u32(&bar_full[g]);
-        if (t > 0) alive = __all_sync(0xffffffffu, wait_cluster(full, (t - 1) & 1, deadp, status));
-        if (!alive) break;
-        if (elect_one()) {
-          if (t > 0 && t + 1 < T) mbar_expect_tx(full, group_bytes(g));
+        for (int g = 0; g < 4; ++g) {
+          const uint32_t full = smem_u32(&bar_full[g]);
+          if (t > 0) {
+            ok = wait_cluster(full, (t - 1) & 1, deadp, status) && ok;
+            if (t + 1 < T && ok) mbar_expect_tx(full, group_bytes(g));
+          }
           tc_fence_after();
 #pragma unroll
           for (int s = g * GS; s < (g + 1) * GS; ++s) {
@@ -445,17 +451,15 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
               }
             }
           }
-          if (g == 3) {
-            umma_commit(smem_u32(&bar_acc));
-            if (t + 1 < T) umma_commit_cluster(smem_u32(&bar_empty), (uint16_t)((1u << C) - 1));
-          }
         }
-        __syncwarp();
+        if (ok) {
+          umma_commit(smem_u32(&bar_acc));
+          if (t + 1 < T) umma_commit_cluster(smem_u32(&bar_empty), (uint16_t)((1u << C) - 1));
+        }
       }
       __syncwarp();
       if (t + 1 < T) {
-        bar_all();                                         // the new slab is staged: one copy to every peer
-        if (__any_sync(0xffffffffu, stopp[t & 1] != 0)) break;
+        if (bar_all_any(!ok)) break;                       // the new slab is staged: one copy to every peer
         if (lane < C) {
           const uint32_t peer = (uint32_t)(rank + lane < C ? rank + lane : rank + lane - C);
           bulk_to_peer(map_to_rank(smem_u32(hbuf) + (uint32_t)lane * SLAB, peer), smem_u32(stg), sent,
@@ -523,7 +527,6 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
       if (t + 1 < T) {
         // every peer has finished reading h_{t-1} (and so has received the slab this buffer held)
         alive = wait_cluster(smem_u32(&bar_empty), t & 1, deadp, status) && alive;
-        if (warp == 0 && !alive) stopp[t & 1] = 1;
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < RPW; ++i) {
@@ -542,8 +545,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
           }
         }
         fence_async_smem();
-        bar_all();
-        if (__any_sync(0xffffffffu, stopp[t & 1] != 0)) break;
+        if (bar_all_any(!alive)) break;
       }
 #pragma unroll
       for (int i = 0; i < RPW; ++i) {
@@ -582,7 +584,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) unsigned long long bar_recv, bar_empty, bar_acc[4];
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead, stop[2], peer_gave_up, unhealthy;
+  __shared__ int dead, peer_gave_up, unhealthy;
   __shared__ float s_fold[ROWS_A], s_scale[ROWS_A];
   __shared__ __align__(16) float s_inv[2][4 * NW];          // inverse row scales of dgh, by step parity
 
@@ -597,7 +599,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   const int RG = (a.rows + 3) >> 2;                        // groups of four rows that are exchanged
   const int u0 = rank * UNITS;
   const int T = a.T;
-  volatile int *deadp = &dead, *stopp = stop;
+  volatile int* deadp = &dead;
   int* status = a.status;
   const uint32_t recv_bytes = (uint32_t)(C * RG * 512);
 
@@ -607,7 +609,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   float* stage = recv + (size_t)C * RG * 128;              // [destination][row group][unit][4 rows]
 
   if (tid == 0) {
-    dead = stop[0] = stop[1] = peer_gave_up = 0;
+    dead = peer_gave_up = 0;
     unhealthy = *reinterpret_cast<volatile int*>(status);
     mbar_init(smem_u32(&bar_recv), 1);
     mbar_init(smem_u32(&bar_empty), C);
@@ -694,7 +696,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
   const size_t row0 = (size_t)(b0 + warp) * H + u;         // first owned element; the others are NW rows apart
   auto fetch = [&](int t) {
     if (t < 0) return;
-    // one base per array: nothing is spilled (a spill misses the little L1 cache that is left beside shared memory)
+    // one base per array keeps the loop's registers down (17 warps leave 96 a thread; -Xptxas -v reports 72 to 136 bytes
+    // spilled in the backward kernels, and a spill can miss the little L1 cache that is left beside shared memory)
     const size_t o = (size_t)t * out_step + row0;
     const float* pd = a.dout + o;
     const float* ps = a.S + o;
@@ -729,8 +732,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
     const uint64_t db0 = desc_sw64(smem_u32(bop), 512);
     const uint64_t da0 = desc_sw64(smem_u32(lo), 512);
     for (int it = 0; it < last; ++it) {
-      bar_all();                                           // dgh of this step is in place
-      if (__any_sync(0xffffffffu, stopp[it & 1] != 0)) break;
+      if (bar_all_any(false)) break;                       // dgh of this step is in place
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
@@ -761,7 +763,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
 #pragma unroll
       for (int i = 0; i < R; ++i) dh[i] = 0.f;
       if (it > 0) {
-        alive = __all_sync(0xffffffffu, wait_cluster(smem_u32(&bar_recv), (it - 1) & 1, deadp, status)) && alive;
+        alive = wait_cluster(smem_u32(&bar_recv), (it - 1) & 1, deadp, status) && alive;
+        __syncwarp();
         if (tid == 0 && it < T && alive) mbar_expect_tx(smem_u32(&bar_recv), recv_bytes);
         // scalar reads of [unit][4 rows]: the rows of a unit are rotated by unit / 8, so that the 32 units of a row
         // lie in 32 banks
@@ -786,8 +789,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
       float gr[R], gz[R], gn[R];
       // the products of the previous step have read the operand (this rank's partial sums may be
       // complete while the last tiles are still under way)
-      if (it > 0) alive = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc[TILES - 1]), (it - 1) & 1, deadp, status)) && alive;
-      if (tid == 0 && !alive) stopp[it & 1] = 1;
+      if (it > 0) alive = mbar_wait(smem_u32(&bar_acc[TILES - 1]), (it - 1) & 1, deadp, status) && alive;
+      __syncwarp();
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         // entries beyond the batch run on zeros, so that the rows of a thread interleave
@@ -819,8 +822,7 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
       // operands of the next step: ahead of the partial sums, behind whose stores a load would queue
       fetch(t - 1);
       fence_async_smem();
-      bar_all();
-      if (__any_sync(0xffffffffu, stopp[it & 1] != 0)) break;
+      if (bar_all_any(!alive)) break;
       // the partial sums of the previous step have been read: peers may overwrite them
       if (it > 0 && warp < C && lane == 0) arrive_at_peer(map_to_rank(smem_u32(&bar_empty), (uint32_t)warp));
       __syncwarp();
@@ -829,8 +831,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
       if (dest < C) {
         bool ready = mbar_wait(smem_u32(&bar_acc[m_own]), it & 1, deadp, status);
         if (it > 0) ready = wait_cluster(smem_u32(&bar_empty), (it - 1) & 1, deadp, status) && ready;
-        ready = __all_sync(0xffffffffu, ready);
         alive = alive && ready;
+        __syncwarp();
         tc_fence_after();
         const uint32_t ts = acc + ((uint32_t)(q_own * 32) << 16) + (uint32_t)(m_own * N);
         const int rot = lane >> 3;
