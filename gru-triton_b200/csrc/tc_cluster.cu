@@ -14,9 +14,11 @@
 //             rank r go to r's receive buffer (bulk copies: st.async stores kept every later load and store of the SM
 //             waiting behind them), r adds the C partials in rank order
 //
-// The fp32 accumulator of the tensor core truncates, so the large products (hi x hi) are summed in
-// two accumulators of at most 16 steps, the small cross products in a third, and the three are added
-// with round-to-nearest.  Integer codes are exact in one (|sum| < 2^24).
+// The fp32 accumulator of the tensor core truncates.  Forward: the leading products (hi x hi) are summed in
+// accumulators of at most 8 steps (16 where the state is on an int8 grid), the small cross products in one of their own,
+// and all are added with round-to-nearest (two of 16 steps: the gradient of b_r at H = 512 was off by 5.4e-7 of 64 bits, 4.5e-7 with four;
+// 5.0e-7 with FP32 FMAs).  Backward: one accumulator per tile, the 12 small products first and the 6 leading ones
+// on top of them (6.7e-7 -> 5.4e-7).  Integer codes are exact in one (|sum| < 2^24).
 //
 // What bounds a step: the exchange.  A CTA receives C slabs at about 15 bytes per cycle over the cluster
 // network (measured; 1300 cycles for the smallest slabs), the products take 12 to 26 cycles per
@@ -221,7 +223,9 @@ template <int N, int CS, int PW, int PH>
 __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
   constexpr int RPW = N / NW;                              // batch rows per compute warp
   constexpr bool EXACT = PW == 1 && PH == 1;
-  constexpr int NACC = EXACT ? 1 : 3;
+  // accumulators of the leading products: eight steps each at most (sixteen on an int8 state, whose grid is far coarser)
+  constexpr int NMAIN = EXACT ? 1 : (CS >= 16 && PH == 2 ? 4 : 2);
+  constexpr int NACC = EXACT ? 1 : NMAIN + 1;
   // Slot i of the operands belongs to rank - i (modulo C), the i-th CTA to send to this one, so that the
   // slabs are consumed in the order in which they arrive.
   // CS slabs (a compile-time count: a branch between two tcgen05.mma costs more than the product, 50
@@ -435,9 +439,9 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
           tc_fence_after();
 #pragma unroll
           for (int s = g * GS; s < (g + 1) * GS; ++s) {
-            // hi x hi: the first half of the positions in the first accumulator, the rest in the second
-            const uint32_t a1 = EXACT ? acc : acc + (uint32_t)((s >= CS / 2 ? 1 : 0) * N), a2 = acc + 2 * N;
-            const bool more = EXACT ? s > 0 : s % (CS / 2) > 0;
+            // the leading products, CS / NMAIN slabs to an accumulator
+            const uint32_t a1 = acc + (uint32_t)(s * NMAIN / CS * N), a2 = acc + NMAIN * N;
+            const bool more = s % (CS / NMAIN) > 0;
             const uint64_t b = dh + (s * SLAB >> 4);
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk) {
@@ -502,10 +506,8 @@ __global__ void __launch_bounds__(NT, 1) tcc_fwd_kernel(const Args a) {
         for (int c = 0; c < CW; ++c) {
           const int b = cg4 * CW + c;
           float v = x[0][c / 4][c % 4];
-          if (!EXACT) {
-            v = v + x[1 % NACC][c / 4][c % 4];
-            v = v + x[2 % NACC][c / 4][c % 4];
-          }
+#pragma unroll
+          for (int p = 1; p < NACC; ++p) v = v + x[p][c / 4][c % 4];
           v = v * wsc;
           if (PH == 2) v = v * s_inv_h[b];
           S[(q * 32 + lane) * LDS + b] = v;
@@ -738,18 +740,20 @@ __global__ void __launch_bounds__(NT, 1) tcc_bwd_kernel(const Args a) {
 #pragma unroll
         for (int m = 0; m < TILES; ++m) {
           const uint32_t d = acc + (uint32_t)(m * N);
+          // one truncating accumulator: the small products first, then six of the leading ones on top of them
 #pragma unroll
           for (int kk = 0; kk < 6; ++kk) {
-            const uint32_t ta = tmem + (uint32_t)(m * 48 + kk * 8);
             const uint64_t b = db0 + (((kk >> 1) * (N * 64) + (kk & 1) * 32) >> 4);
-            umma_ts(d, ta, b, IDESC, kk > 0 ? 1u : 0u);
-            umma_ts(d, ta, b + (PLANE >> 4), IDESC, 1u);
+            umma_ts(d, tmem + (uint32_t)(m * 48 + kk * 8), b + (PLANE >> 4), IDESC, kk > 0 ? 1u : 0u);
             const int blk = m * 3 + (kk >> 1);
             if (PW == 2 && blk < LO_TM)
               umma_ts(d, tmem + (uint32_t)(TILES * 48 + blk * 16 + (kk & 1) * 8), b, IDESC, 1u);
             else if (PW == 2)
               umma<false>(d, da0 + (((blk - LO_TM) * LO_BLK + (kk & 1) * 32) >> 4), b, IDESC, 1u);
           }
+#pragma unroll
+          for (int kk = 0; kk < 6; ++kk)
+            umma_ts(d, tmem + (uint32_t)(m * 48 + kk * 8), db0 + (((kk >> 1) * (N * 64) + (kk & 1) * 32) >> 4), IDESC, 1u);
           umma_commit(smem_u32(&bar_acc[m]));
         }
       }

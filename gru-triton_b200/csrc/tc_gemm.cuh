@@ -47,6 +47,10 @@ int tc_gemm_kblock(const TcGemm& g);
 int tc_gemm_splits(const TcGemm& g, int want);
 int tc_gemm_tile_n(const TcGemm& g);
 int launch_tc_gemm(const TcGemm& g, cudaStream_t st);
+// chunk_kb of the products that carry gradients through weight codes (two planes of dgh or dgi on exact codes): eight
+// steps of the leading product in a chunk instead of sixteen.  Error of such a product 3.4e-7, 7.5e-7 with sixteen; three
+// bf16 planes had 5.1e-7.
+constexpr int TC_GRADIENT_CODES_CHUNK = 2;
 // The same by persistent CTA pairs (tc_gemm2.cu); launch_tc_gemm() checks the arguments and chooses.
 int launch_tc_gemm_pairs(const TcGemm& g, cudaStream_t st);
 

@@ -372,10 +372,10 @@ dh0_kernel(const float* __restrict__ via, int nvia, const float* __restrict__ di
 
 bool codes_fit_int8(const Quant& q) { return q.enabled && q.qmin >= -128.f && q.qmax <= 127.f; }
 
-// plane pairs (i, j) with i + j <= 1, most significant first
+// plane pairs (i, j) with i + j <= 1, the smallest products first: the truncating accumulator loses less on them
 int fill_pairs(int na, int nb, int* pa, int* pb) {
   int n = 0;
-  for (int s = 0; s <= 1; ++s)
+  for (int s = 1; s >= 0; --s)
     for (int i = 0; i <= s; ++i) {
       const int j = s - i;
       if (i < na && j < nb) { pa[n] = i; pb[n] = j; ++n; }
@@ -611,6 +611,7 @@ int launch_tc_dense_backward(const float* h0, const TcWeights& w, const float* o
   gv.lda = 3 * H; gv.ldb = H; gv.a_plane_stride = (long long)B * 3 * H; gv.b_plane_stride = (long long)3 * H * H;
   gv.npairs = fill_pairs(2, p.w_planes, gv.pa, gv.pb);
   gv.split_k = p.via_splits; gv.tile_n = 256;
+  gv.chunk_kb = w.codes != nullptr ? TC_GRADIENT_CODES_CHUNK : 0;
   gv.alpha = 1.0f; gv.row_scale = dgh_inv; gv.C = via; gv.ldc = H; gv.split_stride = (long long)B * H;
 
   // dW[3H,H] (+)= op(dgh)^T[3H,rows] . op(h)[rows,H] over one chunk of time steps
@@ -736,12 +737,7 @@ static TcGemm wgrad_gemm(int T, int B, int H, bool h_codes) {
   g.a_planes = 2; g.b_planes = h_codes ? 1 : 2; g.a_mn = 1; g.b_mn = 1;
   g.lda = 3 * H; g.ldb = H; g.a_plane_stride = rows * 3 * H; g.b_plane_stride = rows * H;
   // two leading planes per fp32 operand and the cross products down to 2^-16: about 5e-6 of a term
-  g.npairs = 0;
-  for (int s2 = 0; s2 <= 1; ++s2)
-    for (int i = 0; i <= s2; ++i) {
-      const int j = s2 - i;
-      if (j < g.b_planes) { g.pa[g.npairs] = i; g.pb[g.npairs] = j; ++g.npairs; }
-    }
+  g.npairs = fill_pairs(g.a_planes, g.b_planes, g.pa, g.pb);
   // wide tiles: one k-block of the two A planes then feeds 256 columns (measured at c1: 31 K cycles
   // per CTA with 256-wide tiles and 4 K slices against 42 K with 128-wide ones)
   g.tile_n = g.N >= 256 ? 256 : 128;
