@@ -245,7 +245,7 @@ static ScanPlan plan_scan(const Dims& d, bool fwd, bool w_codes, const Quant& qi
   double block_cycles = 0.0, tc_cycles = 0.0;
   const bool block = choose_block_config(fwd, d.T, d.B, d.Hb, d.nb, &p.block, &block_cycles);
   const bool tensor = forced != 1 && tcc::choose(fwd, d.T, d.B, d.Hb, d.nb, w_codes, qi, &p.tc, &tc_cycles);
-  p.found = block || tensor;
+  p.found = forced == 2 ? tensor : block || tensor;          // a kernel a test asks for is not replaced by another
   p.tensor = tensor && (forced == 2 || !block || tc_cycles < block_cycles);
   static const bool debug = getenv("B200GRU_DEBUG") != nullptr;
   if (debug)
@@ -616,7 +616,11 @@ int b200gru_test_scan_plan(const b200gru_shape* shape, int backward, int w_codes
   Dims d;
   if (!parse_shape(shape, &d) || plan == nullptr || (d.kind != B200GRU_DENSE && d.kind != B200GRU_MONARCH)) return B200GRU_INVALID_ARGUMENT;
   memset(plan, 0, 6 * sizeof(int));
-  if (step_path(d)) { plan[0] = 3; return B200GRU_OK; }
+  if (step_path(d)) {
+    plan[0] = 3;
+    tc::tc_dense_forward_plan(d.T, d.B, d.H, w_codes != 0, make_quant(q_in), plan + 1, plan + 2);
+    return B200GRU_OK;
+  }
   const ScanPlan p = plan_scan(d, backward == 0, w_codes != 0, make_quant(q_in));
   if (!p.found) return B200GRU_UNSUPPORTED;
   plan[0] = p.tensor ? 2 : 1;

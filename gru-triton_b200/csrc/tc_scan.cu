@@ -451,6 +451,11 @@ bool tc_dense_path(int B, int H) {
   return slice > (size_t)200 * 1024 && B >= 128 && H % 32 == 0;
 }
 
+void tc_dense_forward_plan(int T, int B, int H, bool w_codes, const Quant& qin, int* tile, int* splits) {
+  const Plan p = make_plan(T, B, H, w_codes, qin);
+  *tile = p.i8 ? 0 : p.fwd_tile; *splits = p.i8 ? 1 : p.fwd_splits;
+}
+
 static size_t fwd_scratch(int T, int B, int H, bool w_codes, const Quant& qin) {
   const Plan p = make_plan(T, B, H, w_codes, qin);
   size_t n = 0;

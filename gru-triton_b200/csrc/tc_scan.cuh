@@ -21,6 +21,8 @@ size_t tc_dense_bwd_scratch_bytes(int T, int B, int H, bool w_codes);
 
 int launch_tc_dense_forward(const float* gi, const float* h0, const TcWeights& w, const float* bh, float* out,
                             float* save, void* scratch, int T, int B, int H, Quant qin, Quant qout, cudaStream_t st);
+// Tile width and K slices of the forward product of a step (0 and 1 for the fused int8 step).
+void tc_dense_forward_plan(int T, int B, int H, bool w_codes, const Quant& qin, int* tile, int* splits);
 // dW is the gradient with respect to the weight VALUES (for codes: codes * row_scale).
 int launch_tc_dense_backward(const float* h0, const TcWeights& w, const float* out, const float* S, const float* dout,
                              float* dgi, float* dh0, float* dW, float* dbh, float* dbi, void* scratch, int T, int B, int H,

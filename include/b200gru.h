@@ -329,11 +329,12 @@ int b200gru_calibration_scan(const b200gru_shape* shape, const float* gi, const 
  * kernels, resp. the diagonal forward use its register-ring kernel, on every shape, so that the
  * tests can hold both to the same parity bar.  Process-wide; (0, 0) restores the normal dispatch.
  * b200gru_test_select_dense_scan: 1 makes dense / block-diagonal scans use the FP32 cluster kernels,
- * 2 the tensor-core cluster scan wherever it applies; 0 restores the choice by shape.
- * b200gru_test_select_gemm: 1 makes the tensor-core products use single CTAs, 2 pairs of CTAs; 0 the
- * choice by shape.
+ * 2 the tensor-core cluster scan (UNSUPPORTED where it does not apply); 0 restores the choice by shape.
+ * b200gru_test_select_gemm: 1 makes the tensor-core products use single CTAs, 2 pairs of CTAs (UNSUPPORTED where
+ * they do not apply); 0 the choice by shape.
  * b200gru_test_scan_plan: the kernel of a dense / block-diagonal scan as plan[0] (1 FP32 clusters, 2 tensor-core clusters,
- * 3 one product per step); for 2 its CTAs per cluster, row tile, rows per cluster, clusters and dynamic shared memory.
+ * 3 one product per step); for 2 its CTAs per cluster, row tile, rows per cluster, clusters and dynamic shared memory;
+ * for 3 the tile width and K slices of the forward product.
  * b200gru_test_set_scan_status: writes the status word of the tensor-core cluster scans, as a wait that ran out would.
  * b200gru_test_wait_timeout: launches one tiny kernel whose bounded wait must run out (it waits
  * about a millisecond for bytes nothing sends), which sets the flag b200gru_device_status

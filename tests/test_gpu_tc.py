@@ -746,3 +746,90 @@ def test_layer_error_against_64_bits(kind, T, B, H, wbits):
     error = lambda a, b: float((a.detach().double() - b.detach()).norm() / b.detach().norm())
     print("out %.2e dx %.2e" % (error(out, want), error(xg.grad, xr.grad)))
     assert error(out, want) <= (5.3e-7 if wbits == 8 else 5e-7) and error(xg.grad, xr.grad) <= (8e-7 if wbits == 8 else 5e-7)
+
+
+# ---- the same against 64 bits, over sizes that take other branches ---------------------------------------
+
+
+@pytest.mark.parametrize("wbits", [32, 8])
+@pytest.mark.parametrize("T,B", [(1, 32769), (4, 8200), (3, 21900)])
+def test_layer_entry_over_several_row_chunks(T, B, wbits):
+    """Operand planes exist for 32768 rows at a time: one row more, a short second chunk, three chunks.  Gradients that
+    accumulate over the chunks, and K slices that the short chunk has fewer of, against the layer in 64 bits."""
+    layer = _layer(40, 64, wbits=wbits)
+    _grid_weights(layer)
+    ref = copy.deepcopy(layer).double()
+    ref.use_triton = False
+    g = torch.Generator(device="cuda").manual_seed(B)
+    x, h0, dout = (torch.randn(s, device="cuda", generator=g) for s in ((T, B, 40), (B, 64), (T, B, 64)))
+    results = []
+    for l, cast in ((layer, torch.Tensor.float), (ref, torch.Tensor.double)):
+        xg, hg = cast(x).clone().requires_grad_(True), cast(h0 * 0.1).requires_grad_(True)
+        out, _ = l(xg, hg)
+        out.backward(cast(dout))
+        results.append([out.detach(), xg.grad, hg.grad] + [p.grad for p in l.parameters()])
+    (got, *grads), (want, *wants) = results
+    assert bool(((got.double() - want).abs() <= FWD_TOL + FWD_TOL * want.abs()).all())
+    for a, b in zip(grads, wants):
+        assert rel_err(a, b) <= GRAD_TOL
+
+
+def _dense64(gi, h0, W, bh):
+    """The unquantised dense scan in the precision of its arguments, by plain torch operations."""
+    h, outs = h0, []
+    for t in range(gi.shape[0]):
+        gr, gz, gn = gi[t].chunk(3, -1)
+        hr, hz, hn = (h @ W.t() + bh).chunk(3, -1)
+        z, n = torch.sigmoid(gz + hz), torch.tanh(gn + torch.sigmoid(gr + hr) * hn)
+        h = (1 - z) * n + z * h
+        outs.append(h)
+    return torch.stack(outs)
+
+
+@pytest.mark.parametrize("T,B,H", [(2, 128, 4128), (2, 130, 4064), (3, 256, 1024), (3, 300, 1024), (3, 1100, 1024), (4, 129, 544)])
+def test_step_path_against_64_bits(T, B, H):
+    """One product per step: rows with more groups of four than a block has threads (H > 4096), the widest row that has
+    not, and batches whose forward product takes different numbers of K slices."""
+    from gru_triton_b200 import _lib
+    assert _scan_plan(T, B, H)[0] == 3
+    g = torch.Generator(device="cuda").manual_seed(H + B)
+    gi, h0, dout = (torch.randn(s, device="cuda", generator=g) for s in ((T, B, 3 * H), (B, H), (T, B, H)))
+    W = (torch.rand(3 * H, H, device="cuda", generator=g) * 2 - 1) * H ** -0.5
+    bh = torch.randn(3 * H, device="cuda", generator=g) * 0.1
+    out, save = _lib.scan_forward("dense", gi, h0, W, bh, None, None, want_save=True)
+    grads = _lib.scan_backward("dense", gi, h0, W, bh, out, dout, save, None, None)
+    leaves = [t.double().requires_grad_(True) for t in (gi, h0, W, bh)]
+    want = _dense64(*leaves)
+    assert bool(((out.double() - want).abs() <= FWD_TOL + FWD_TOL * want.abs()).all())
+    for a, b in zip(grads, torch.autograd.grad(want, leaves, dout.double())):
+        assert rel_err(a, b) <= GRAD_TOL
+
+
+def test_step_path_slices_differ():
+    """What the case above relies on: the batches of H = 1024 have one, two and three K slices."""
+    assert len({_scan_plan(3, B, 1024)[2] for B in (256, 300, 1100)}) >= 2
+
+
+@pytest.mark.parametrize("size", [1.0, 1e3, 1e5])
+@pytest.mark.parametrize("B,H", [(5, 96), (40, 512), (128, 608)])
+def test_state_that_starts_far_outside_the_unit_range(B, H, size):
+    """The state's fp16 planes are relative to max(1, |h0|) of the row for the whole scan; up to |h0| = 2^17 a state that
+    has decayed to 1 still has its 22 bits.  Every step after the first from the device's own previous state."""
+    from gru_triton_b200 import _lib
+    T = 4
+    g = torch.Generator(device="cuda").manual_seed(H)
+    gi, h0 = (torch.randn(s, device="cuda", generator=g) for s in ((T, B, 3 * H), (B, H)))
+    gi[0, :, H:2 * H] = -30.0                                  # the first step forgets h0
+    W = (torch.rand(3 * H, H, device="cuda", generator=g) * 2 - 1) * H ** -0.5
+    bh = torch.zeros(3 * H, device="cuda")
+    W[H:2 * H] *= 1e-9
+    _lib.load().b200gru_test_select_dense_scan(2 if B < 128 else 0)
+    try:
+        out, _ = _lib.scan_forward("dense", gi, h0 * size, W, bh, None, None)
+        torch.cuda.synchronize()
+    finally:
+        _lib.load().b200gru_test_select_dense_scan(0)
+    assert bool((out.abs() <= 1.0 + 1e-6).all())
+    for t in range(1, T):
+        want = _dense64(gi[t:t + 1].double(), out[t - 1].double(), W.double(), bh.double())[0]
+        assert float((out[t].double() - want).abs().max()) <= FWD_TOL
