@@ -833,3 +833,29 @@ def test_state_that_starts_far_outside_the_unit_range(B, H, size):
     for t in range(1, T):
         want = _dense64(gi[t:t + 1].double(), out[t - 1].double(), W.double(), bh.double())[0]
         assert float((out[t].double() - want).abs().max()) <= FWD_TOL
+
+
+# ---- what a row's result depends on -------------------------------------------------------------------------
+
+@pytest.mark.parametrize("H", [64, 128, 512, 1024])
+def test_a_row_in_other_batches(H):
+    """The kernel of a dense scan, and the K slices of its products, are chosen by T and B: a row's forward result is
+    the same to rounding in every batch, not bit for bit.  In each it is within the forward bar of 64 bits, and the
+    same call repeats its bits."""
+    from gru_triton_b200 import _lib
+    T, by_plan = 12, {}
+    for B in (1, 2, 4, 8, 16, 32, 64, 100, 256, 300, 600, 1100):
+        plan = _scan_plan(T, B, H)
+        by_plan.setdefault(plan[:1] if plan[0] < 3 else plan[:3], B)
+    assert H == 512 or len(by_plan) > 1                        # the batches lie on both sides of a choice
+    most = max(by_plan.values())
+    g = torch.Generator(device="cuda").manual_seed(H)
+    gi, h0 = torch.randn(T, most, 3 * H, device="cuda", generator=g), torch.randn(most, H, device="cuda", generator=g)
+    W = (torch.rand(3 * H, H, device="cuda", generator=g) * 2 - 1) * H ** -0.5
+    bh = torch.zeros(3 * H, device="cuda")
+    want = _dense64(gi[:, :1].double(), h0[:1].double(), W.double(), bh.double())
+    for B in by_plan.values():
+        run = lambda: _lib.scan_forward("dense", gi[:, :B].contiguous(), h0[:B].contiguous(), W, bh, None, None)[0]
+        out = run()
+        assert torch.equal(out, run())
+        assert bool(((out[:, :1].double() - want).abs() <= FWD_TOL + FWD_TOL * want.abs()).all())
