@@ -998,10 +998,14 @@ bool choose_block_config(bool fwd, int T, int B, int Hb, int nb, BlockScanConfig
         const double wstream = 3.0 * Hc4 * Hb * 4.0 / (ws ? 128.0 : 24.0), hstream = (double)Hb * BT * 4.0 * NW / 128.0;
         double step;
         if (fwd) {
-          step = 0.6 * wstream + fma + hstream + (200.0 + 290.0 * BT) * ipw + (C > 1 ? 700.0 + 40.0 * C : (ipw > 1 ? 1000.0 : 700.0));
+          // Hb = 128, C = 8 and 4: 1780 and 1940 cycles; Hb = 256, C = 16 and 8: 1970 and 2180; Hb = 192, C = 4 (two items a warp): 3550
+          step = 0.6 * wstream + fma + hstream + (200.0 + 290.0 * BT) * ipw * (C > 1 && ipw > 1 ? 1.6 : 1.0) +
+                 (C > 1 ? 985.0 + 10.0 * C : (ipw > 1 ? 1000.0 : 700.0));
         } else {
           const double barrier = C > 1 ? 1200.0 + 40.0 * C : 1200.0;
           step = (fma > wstream + hstream ? fma : wstream + hstream) + barrier + 400.0;
+          // more tiles of 32 positions than warps: the contraction runs twice (Hb = 384: 530 us of 200 steps, Hb = 512 449)
+          if (c.TW == 1 && ntiles > NW) step += fma > wstream + hstream ? fma : wstream + hstream;
           step += c.TW == 1 ? 45.0 * Hc4 * (BT - 1) / c.NH : 0.11 * (BT - 1) * step;
         }
         const double setup = fwd ? 8000.0 + 1100.0 * C : 11500.0 + 530.0 * C;       // launch, weight slice

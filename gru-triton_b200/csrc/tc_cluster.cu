@@ -1003,12 +1003,21 @@ bool choose(bool fwd, int T, int B, int Hb, int nb, bool w_codes, const Quant& q
     }
     const long long clusters = (long long)nb * cdiv(B, rows);
     const double waves = (double)((clusters + active - 1) / active);
-    // Cycles of a step as measured over C = 2 .. 16 and 1 .. 37 rows (within 15 %): a fixed part, the gate work of
+    // Cycles of a step as measured over C = 1 .. 16 and 1 .. 43 rows (within 15 %): a fixed part, the gate work of
     // 16 rows, and per CTA of the cluster one bulk copy and its bytes (the backward shares the SM's outgoing
-    // port with dgi and is slower).  H = 512: forward 4250 at 5 rows and 10700 at 37; backward 5400 at 5, 9000 at 19.
+    // port with dgi and is slower).  H = 512: forward 4700 at 4 rows and 11700 at 43; backward 5400 at 5, 9000 at 19.
+    // With few rows the forward is bound by issuing the products of its CS slabs: 2500 cycles at 4 slabs, 4700 at 16
+    // (int8 state: 2350 and 3950; integer codes of both operands fewer still).  The backward of small clusters lies above
+    // its exchange as well: with 300 rows of 64 units it takes 736 us where the FP32 kernel takes 640.
+    static const double least[3][3] = {{2500.0, 2950.0, 4650.0}, {2350.0, 2750.0, 3900.0}, {2100.0, 2400.0, 3400.0}};
     const double slab = fwd ? (double)ph * ((rows + 7) / 8 * 8) * 64 : (double)((rows + 3) / 4) * 512;
-    const double step = fwd ? 750.0 + C * (60.0 + slab / 15.0) + 1000.0 * (N / 16)
-                            : 1300.0 + C * (50.0 + slab / 8.3) + 1000.0 * (N / 16);
+    double step = fwd ? 750.0 + C * (60.0 + slab / 15.0) + 1000.0 * (N / 16) : 1300.0 + C * (50.0 + slab / 8.3) + 1000.0 * (N / 16);
+    if (fwd) {
+      const double low = least[pw == 1 ? 2 : 2 - ph][cs / 8] + 1000.0 * (N / 16 - 1);
+      if (step < low) step = low;
+    } else if (cs == 4) {
+      step *= 1.3;
+    }
     // set-up (weights into tensor memory), from T = 1 and T = 4 launches
     const double setup = fwd ? 12000.0 + 750.0 * C : 18500.0 + 850.0 * C;
     const double cost = waves * (step * T + setup);

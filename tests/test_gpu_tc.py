@@ -859,3 +859,12 @@ def test_a_row_in_other_batches(H):
         out = run()
         assert torch.equal(out, run())
         assert bool(((out[:, :1].double() - want).abs() <= FWD_TOL + FWD_TOL * want.abs()).all())
+
+
+@pytest.mark.parametrize("T,B,H,nb,backward,quant,kernel", [
+    (200, 4, 512, 1, False, True, 1), (200, 1, 512, 1, False, False, 1), (200, 36, 192, 16, False, False, 1), (200, 150, 48, 4, False, False, 1),
+    (200, 32, 192, 1, False, False, 2), (64, 32, 512, 1, False, False, 2), (64, 256, 512, 1, False, False, 2), (200, 300, 128, 1, False, True, 2),
+    (200, 300, 64, 1, True, False, 1), (30, 12, 384, 1, True, False, 2), (64, 256, 512, 1, True, False, 2)])
+def test_dense_scan_dispatch(T, B, H, nb, backward, quant, kernel):
+    """The kernel that measures faster by at least 8 % (FP32 clusters 1, tensor-core clusters 2) is the one chosen."""
+    assert _scan_plan(T, B, H, nb, backward=backward, quant=(1 / 127.0, -127, 127) if quant else None)[0] == kernel
