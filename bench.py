@@ -54,7 +54,7 @@ CONFIGS = {
 ROOFLINE_TRAFFIC = {
     "c1": dict(bytes=15.86e6, T=64),
     "c2": dict(bytes=512.6e6, T=128),
-    "c3": dict(bytes=13.11e6, T=64),
+    "c3": dict(bytes=13.09e6, T=64),
     "c4": dict(bytes=212.7e6, T=128),
 }
 # config 5: one launch of the fused forward step at B = 512 rows per GPU (profiles/): 3.15 MB of weight
@@ -321,8 +321,20 @@ def load_peaks():
     return json.load(open(ppath)) if os.path.exists(ppath) else {}
 
 
+def scan_kernel(cfg, T, B, H):
+    """Name of the forward-scan kernel that the library chooses for a dense or block-diagonal shape."""
+    import ctypes
+
+    from gru_triton_b200 import _lib
+    plan = (ctypes.c_int * 6)()
+    shape = _lib.make_shape(cfg["kind"], T, B, H, cfg.get("nblocks", 1))
+    quant = _lib._cquant((1 / 127.0, -127, 127) if cfg["quant"] else None)
+    rc = _lib.load().b200gru_test_scan_plan(ctypes.byref(shape), 0, int(cfg.get("wbits", 32) <= 8), ctypes.byref(quant), plan)
+    return {1: "block_fwd_kernel", 2: "tcc_fwd_kernel"}.get(plan[0], "unknown") if rc == 0 else "unknown"
+
+
 def tensor_roofline(wl, k_ms, scan_launches, peaks):
-    """Forward scan of the tensor-core path: T products [B,H] x [H,3H], int8 codes (exact) or bf16
+    """Forward scan of the tensor-core path: T products [B,H] x [H,3H], int8 codes (exact) or fp16
     planes, against the measured sustained bf16 GEMM rate."""
     flops = 2.0 * wl.T * wl.B * wl.H * 3 * wl.H
     peak_tf = float(peaks.get("bf16_tflops_sustained", 1400.0))
@@ -511,8 +523,8 @@ def run_device(args):
         fp32_peak = 148 * 128 * 2 * 1.965e9 / 1e12          # FMA lanes x 2 flops x max SM clock, nominal
         scan_flops = {"dense": 6.0 * Hm * Hm, "monarch": 6.0 * Hm * (Hm // cfg.get("nblocks", 4)),
                       "butterfly": 9.0 * Hm * max(1, (Hm - 1).bit_length()), "diagonal": 40.0 * Hm}[cfg["kind"]] * Tm * Bm
-        roofline = {"kernel": {"dense": "block_fwd_kernel", "monarch": "block_fwd_kernel",
-                               "diagonal": "diag_fwd_tma_kernel", "butterfly": "bfly_fwd2_kernel"}[cfg["kind"]],
+        roofline = {"kernel": {"diagonal": "diag_fwd_tma_kernel", "butterfly": "bfly_fwd2_kernel"}.get(cfg["kind"])
+                              or scan_kernel(cfg, Tm, Bm, Hm),
                     "bound": "latency" if latency_bound else "hbm",
                     "achieved": achieved, "peak": peak_gbs, "unit": "GB/s",
                     "frac": achieved / peak_gbs, "peak_source": "measured" if peaks else "fallback",
